@@ -1,156 +1,406 @@
-// plain.cu -- the plain FP32 chain: one kernel per stage, the reference's
-// scalar method (Gram, coef_apply, LLR) plus the FP32 Cholesky MMSE solve the
-// reference lacks.  Every stage is bit-exact with the CPU restatement in the
-// checker because each output element is accumulated in the same order with
-// the same fused multiply-adds.
+// plain.cu -- the plain FP32 chain: the reference's scalar method (Gram,
+// coef_apply, LLR) plus the FP32 Cholesky MMSE solve the reference lacks, stage
+// by stage or as one kernel.  Every stage is bit-exact with the CPU restatement
+// in the checker because each output element is accumulated in the same order
+// with the same fused multiply-adds.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace aeq {
 
 // ---------------------------------------------------------------------------
-// Gram: G[sc][r][c] = sum_k cma(conj(H[k][r]), H[k][c]) (+ sigma2 if r == c).
-// gram_scalar (src/aerial_bottleneck.cu:56-80) with M = H^H; one thread per
-// output element, the antenna sum in order.
+// One kernel for every stage but the stand-alone demapper.  A team of TEAM
+// lanes owns a subcarrier; its H, Y and C sit in shared memory, G and the
+// trailing block of the factor in registers.
+//
+//   kGram   H -> G                       gram_scalar (src/aerial_bottleneck.cu:56-80), M = H^H
+//   kCoef   G, H -> C, noiseInv          the FP32 Cholesky MMSE solve
+//   kApply  C, Y -> Y_eq                 coef_apply_v1_scalar (src/aerial_coef_wmma.cu:71-104)
+//   kChain  H, Y -> LLR (and Y_eq)       all of them and the demapper; G, C and noiseInv
+//                                        never leave the SM
+//
+// Every value is accumulated in the serial specification's order with its
+// fused multiply-adds; lanes only divide the values among themselves:
+//   G       lane: row r, columns 2p, 2p + 1, antennas in order.
+//   factor  column by column, right-looking: the lane that holds (i, j) takes
+//           L_ik conj(L_jk) off it at step k = 0, 1, ..., which is the order
+//           of the left-looking sum.
+//   C       lane: antennas tid, tid + TEAM, ... (two at a time, for two
+//           independent chains); forward and backward substitution in registers.
+//   mu      lane l: sum over the antennas in order.
+//   Y_eq    lane: one layer and up to TS symbols, antennas in order.
+//
+// What bounds it: the FMA and shared-memory pipes at about equal shares.  A
+// thread per output element, as the reference has it, reads two operands from
+// L1 for each complex product; here a lane's operands serve two columns (G)
+// or up to four symbols (Y_eq) from one 16-byte read each, rows are padded so
+// that a warp's reads meet no bank conflicts, and the intermediates' 27.6 MB
+// per 100 MHz slot of HBM traffic are gone from the chain.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) gram_kernel(const cf* __restrict__ H, float sigma2,
-                                                    cf* __restrict__ G, long total, int A, int L) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    int c = (int)(t % L);
-    int r = (int)((t / L) % L);
-    long sc = t / ((long)L * L);
-    const cf* h = H + sc * (long)A * L;
-    cf acc = make_float2(0.f, 0.f);
-    for (int k = 0; k < A; k++) {
-        cf m = __ldg(&h[k * L + r]);
-        m.y = -m.y;
-        acc = cma(m, __ldg(&h[k * L + c]), acc);
-    }
-    if (r == c) acc.x = __fadd_rn(acc.x, sigma2);
-    G[t] = acc;
+enum PlainMode : int { kGram = 0, kCoef = 1, kApply = 2, kChain = 3 };
+
+struct PlainCell {
+    const cf* H;
+    const cf* Y;
+    cf* G;              // kGram: out, kCoef: in
+    cf* C;              // kCoef: out, kApply: in
+    float* nInv;        // kCoef: out
+    cf* O;              // kApply: out, kChain: optional out
+    float* llr;
+    float sigma2;
+    int nSC, A, L, S, nPam;
+    int vecH, vecY;     // 16-byte rows of H (L even, aligned); of Y and C (A even, aligned)
+    unsigned block0;    // first block of this cell
+    PamLut lut;
+};
+struct PlainParams {
+    PlainCell cell[AERIAL_MAX_CELLS];
+    int nCells;
+    int teamBytes;      // shared memory per team
+};
+
+// Lanes per subcarrier: 16 for up to 4 layers, a warp for 8, four warps for
+// 16 (whose factor has 72 column pairs and whose C needs 128 antennas' worth
+// of lanes to keep the FMA pipe fed at two or three resident blocks per SM).
+__host__ __device__ constexpr int plain_team(int LT) { return LT <= 4 ? 16 : LT == 8 ? 32 : 128; }
+
+// Row strides in complex values: even (16-byte rows) and 16 bytes past a
+// multiple of the row, so that eight rows read at once differ in banks.
+__host__ __device__ __forceinline__ int plain_hs(int L) { return ((L + 1) & ~1) + 2; }
+__host__ __device__ __forceinline__ int plain_cs(int A) { return ((A + 1) & ~1) + 2; }
+
+static int plain_team_bytes(int mode, int A, int L, int S) {
+    int v = 0;
+    if (mode != kApply) v += A * plain_hs(L);
+    if (mode != kGram) v += L * plain_cs(A);
+    if (mode == kApply || mode == kChain) v += S * plain_cs(A);
+    if (mode == kCoef || mode == kChain) v += L * L + ((3 * L + 1) / 2 + 1);
+    return ((v + 1) & ~1) * (int)sizeof(cf);
 }
 
-// ---------------------------------------------------------------------------
-// MMSE coefficients.  One block per subcarrier.
-//   1. Cholesky G = Lc Lc^H, column by column; thread i computes Lc[i][j]
-//      (its whole sum in order), so the arithmetic is the serial
-//      specification's.
-//   2. Thread a solves G x = conj(H[a][:]) -> column a of C.
-//   3. Thread l sums mu_l = Re sum_a C[l][a] H[a][l] in antenna order.
-//   4. C[l][:] *= 1/mu_l; noiseInv[l] = mu_l / (1 - mu_l).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) mmse_coef_kernel(const cf* __restrict__ G,
-                                                         const cf* __restrict__ H, cf* __restrict__ C,
-                                                         float* __restrict__ noiseInv, int A, int L) {
-    extern __shared__ float2 sm[];
-    cf* sL = sm;                  // [L][L]
-    cf* sX = sm + L * L;          // [L][A]
-    float* sInv = (float*)(sX + (long)L * A);   // [L]
-    float* sMuInv = sInv + L;                    // [L]
-    const long sc = blockIdx.x;
-    const cf* g = G + sc * L * L;
-    const cf* h = H + sc * (long)A * L;
-    const int tid = threadIdx.x;
+template <int TEAM>
+__device__ __forceinline__ void team_sync() {
+    if constexpr (TEAM > 32) __syncthreads();
+    else __syncwarp();
+}
+__device__ __forceinline__ uint32_t sm_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp16(cf* d, const cf* s) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sm_addr(d)), "l"(__cvta_generic_to_global(s))
+                 : "memory");
+}
+__device__ __forceinline__ void cp8(cf* d, const cf* s) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sm_addr(d)), "l"(__cvta_generic_to_global(s))
+                 : "memory");
+}
+__device__ __forceinline__ float4 ld4(const cf* p) { return *reinterpret_cast<const float4*>(p); }
 
-    for (int j = 0; j < L; j++) {
-        if (tid == 0) {
-            float s = g[j * L + j].x;
-            for (int k = 0; k < j; k++) {
-                cf x = sL[j * L + k];
-                s = __fmaf_rn(-x.x, x.x, s);
-                s = __fmaf_rn(-x.y, x.y, s);
+// rows x cols values of src (contiguous) into rows of stride ds.
+template <int TEAM>
+__device__ __forceinline__ void stage_rows(cf* dst, int ds, const cf* src, int rows, int cols, int vec, int tid) {
+    if (vec) {
+        const int half = cols >> 1;
+        if (half >= TEAM) {
+            for (int r = 0; r < rows; r++)
+                for (int k = tid; k < half; k += TEAM) cp16(dst + r * ds + 2 * k, src + (long)r * cols + 2 * k);
+        } else {
+            for (int e = tid; e < rows * half; e += TEAM) {
+                const int r = e / half, k = e - r * half;
+                cp16(dst + r * ds + 2 * k, src + 2 * e);
             }
-            if (!(s > 0.f)) s = 1e-30f;
-            float d = __fsqrt_rn(s);
-            sInv[j] = __fdiv_rn(1.0f, d);
-            sL[j * L + j] = make_float2(d, 0.f);
         }
-        __syncthreads();
-        const float iv = sInv[j];
-        for (int i = j + 1 + tid; i < L; i += blockDim.x) {
-            cf acc = g[i * L + j];
-            for (int k = 0; k < j; k++) {
-                cf a = sL[i * L + k], b = sL[j * L + k];
-                acc.x = __fmaf_rn(-a.x, b.x, acc.x);
-                acc.x = __fmaf_rn(-a.y, b.y, acc.x);
-                acc.y = __fmaf_rn(-a.y, b.x, acc.y);
-                acc.y = __fmaf_rn(a.x, b.y, acc.y);
-            }
-            sL[i * L + j] = make_float2(__fmul_rn(acc.x, iv), __fmul_rn(acc.y, iv));
+    } else {
+        for (int e = tid; e < rows * cols; e += TEAM) {
+            const int r = e / cols;
+            cp8(dst + r * ds + (e - r * cols), src + e);
         }
-        __syncthreads();
     }
+}
 
-    for (int a = tid; a < A; a += blockDim.x) {
-        cf w[AERIAL_MAX_LAYERS], x[AERIAL_MAX_LAYERS];
-        for (int i = 0; i < L; i++) {
-            cf hv = __ldg(&h[a * L + i]);
-            cf acc = make_float2(hv.x, -hv.y);
-            for (int k = 0; k < i; k++) {
-                cf lv = sL[i * L + k], y = w[k];
+// C columns of NA antennas a, a + TEAM: G x = conj(H[a][:]).
+template <int LT, bool EX, int NA, int TEAM>
+__device__ __forceinline__ void solve_antennas(const cf* sH, int hs, const cf* sL, const float* sInv, cf* sC, int cs,
+                                               int L, int a) {
+    cf w[NA][LT];
+#pragma unroll
+    for (int n = 0; n < NA; n++) {
+        const cf* h = sH + (a + n * TEAM) * hs;
+#pragma unroll
+        for (int i = 0; i < LT; i += 2) {
+            if (!EX && i >= L) break;
+            const float4 v = ld4(h + i);
+            w[n][i] = make_float2(v.x, -v.y);
+            w[n][i + 1] = make_float2(v.z, -v.w);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < LT; i++) {
+        if (!EX && i >= L) break;
+#pragma unroll
+        for (int k = 0; k < i; k++) {
+            const cf lv = sL[i * L + k];
+#pragma unroll
+            for (int n = 0; n < NA; n++) {
+                const cf y = w[n][k];
+                cf& acc = w[n][i];
                 acc.x = __fmaf_rn(-lv.x, y.x, acc.x);
                 acc.x = __fmaf_rn(lv.y, y.y, acc.x);
                 acc.y = __fmaf_rn(-lv.x, y.y, acc.y);
                 acc.y = __fmaf_rn(-lv.y, y.x, acc.y);
             }
-            w[i] = make_float2(__fmul_rn(acc.x, sInv[i]), __fmul_rn(acc.y, sInv[i]));
         }
-        for (int i = L - 1; i >= 0; i--) {
-            cf acc = w[i];
-            for (int k = i + 1; k < L; k++) {
-                cf lv = sL[k * L + i], y = x[k];
+        const float iv = sInv[i];
+#pragma unroll
+        for (int n = 0; n < NA; n++) w[n][i] = make_float2(__fmul_rn(w[n][i].x, iv), __fmul_rn(w[n][i].y, iv));
+    }
+#pragma unroll
+    for (int i = LT - 1; i >= 0; i--) {
+        if (!EX && i >= L) continue;
+#pragma unroll
+        for (int k = i + 1; k < LT; k++) {
+            if (!EX && k >= L) break;
+            const cf lv = sL[k * L + i];
+#pragma unroll
+            for (int n = 0; n < NA; n++) {
+                const cf y = w[n][k];
+                cf& acc = w[n][i];
                 acc.x = __fmaf_rn(-lv.x, y.x, acc.x);
                 acc.x = __fmaf_rn(-lv.y, y.y, acc.x);
                 acc.y = __fmaf_rn(-lv.x, y.y, acc.y);
                 acc.y = __fmaf_rn(lv.y, y.x, acc.y);
             }
-            x[i] = make_float2(__fmul_rn(acc.x, sInv[i]), __fmul_rn(acc.y, sInv[i]));
         }
-        for (int l = 0; l < L; l++) sX[l * A + a] = x[l];
-    }
-    __syncthreads();
-    for (int l = tid; l < L; l += blockDim.x) {
-        float mu = 0.f;
-        for (int a = 0; a < A; a++) {
-            cf c = sX[l * A + a], hv = __ldg(&h[a * L + l]);
-            mu = __fmaf_rn(c.x, hv.x, mu);
-            mu = __fmaf_rn(-c.y, hv.y, mu);
+        const float iv = sInv[i];
+#pragma unroll
+        for (int n = 0; n < NA; n++) {
+            w[n][i] = make_float2(__fmul_rn(w[n][i].x, iv), __fmul_rn(w[n][i].y, iv));
+            sC[i * cs + a + n * TEAM] = w[n][i];
         }
-        sMuInv[l] = __fdiv_rn(1.0f, mu);
-        noiseInv[sc * L + l] = __fdiv_rn(mu, __fsub_rn(1.0f, mu));
-    }
-    __syncthreads();
-    cf* c = C + sc * (long)L * A;
-    for (int e = tid; e < L * A; e += blockDim.x) {
-        cf v = sX[e];
-        float im = sMuInv[e / A];
-        c[e] = make_float2(__fmul_rn(v.x, im), __fmul_rn(v.y, im));
     }
 }
 
-// ---------------------------------------------------------------------------
-// coef_apply, coef_apply_v1_scalar (src/aerial_coef_wmma.cu:71-104): grid
-// (PRBs, layers), block (12 subcarriers, nSym); C[sc][layer][:] staged in
-// shared memory; each thread sums its antenna products in order.
-// ---------------------------------------------------------------------------
-__global__ void coef_apply_kernel(const cf* __restrict__ C, const cf* __restrict__ Y,
-                                  cf* __restrict__ O, int nSC, int nSym, int L, int A) {
-    extern __shared__ float2 sC[];  // [A][12]
-    const int prb = blockIdx.x, layer = blockIdx.y;
-    const int scl = threadIdx.x, sym = threadIdx.y;
-    const int sc = prb * 12 + scl;
-    const int nt = blockDim.x * blockDim.y;
-    for (int e = threadIdx.y * blockDim.x + threadIdx.x; e < A * 12; e += nt) {
-        int s2 = e / A, a = e % A;
-        int scc = prb * 12 + s2;
-        if (scc < nSC) sC[a * 12 + s2] = __ldg(&C[((long)scc * L + layer) * A + a]);
+template <int N>
+__device__ __forceinline__ void plain_llr_store(cf v, float noise, const PamLut& lut, float* dst) {
+    float o[2 * N];
+    pam_llr<N>(v.x, v.y, noise, lut, o);
+    // rows of 8 N bytes from an 8-byte aligned array
+#pragma unroll
+    for (int j = 0; j < 2 * N; j += 2) *reinterpret_cast<float2*>(dst + j) = make_float2(o[j], o[j + 1]);
+}
+
+// Y_eq of layer l, symbols st, st + LPL, ... (TS of them; those past S are
+// computed on row 0 and dropped).
+template <int MODE, int TS, int LPL>
+__device__ __forceinline__ void apply_symbols(const PlainCell& cl, const cf* sC, const cf* sY, int cs, float noise,
+                                              long sc, int l, int st, bool out) {
+    const int A = cl.A, S = cl.S, L = cl.L;
+    const cf* c = sC + l * cs;
+    const cf* y[TS];
+    cf acc[TS];
+#pragma unroll
+    for (int t = 0; t < TS; t++) {
+        const int s = st + t * LPL;
+        y[t] = sY + (s < S ? s : 0) * cs;
+        acc[t] = make_float2(0.f, 0.f);
     }
-    __syncthreads();
-    if (sc >= nSC || sym >= nSym) return;
-    const cf* y = Y + ((long)sc * nSym + sym) * A;
-    cf acc = make_float2(0.f, 0.f);
-    for (int a = 0; a < A; a++) acc = cma(sC[a * 12 + scl], __ldg(&y[a]), acc);
-    O[((long)sc * L + layer) * nSym + sym] = acc;
+    int a = 0;
+#pragma unroll 2
+    for (; a + 1 < A; a += 2) {
+        const float4 cv = ld4(c + a);
+        float4 yv[TS];
+#pragma unroll
+        for (int t = 0; t < TS; t++) yv[t] = ld4(y[t] + a);
+#pragma unroll
+        for (int t = 0; t < TS; t++) acc[t] = cma(make_float2(cv.x, cv.y), make_float2(yv[t].x, yv[t].y), acc[t]);
+#pragma unroll
+        for (int t = 0; t < TS; t++) acc[t] = cma(make_float2(cv.z, cv.w), make_float2(yv[t].z, yv[t].w), acc[t]);
+    }
+    if (a < A) {
+#pragma unroll
+        for (int t = 0; t < TS; t++) acc[t] = cma(c[a], y[t][a], acc[t]);
+    }
+    const long row = (sc * L + l) * (long)S;
+#pragma unroll
+    for (int t = 0; t < TS; t++) {
+        const int s = st + t * LPL;
+        if (!out || s >= S) continue;
+        if (MODE == kApply || cl.O) cl.O[row + s] = acc[t];
+        if constexpr (MODE == kChain) {
+            float* dst = cl.llr + (row + s) * 2 * cl.nPam;
+            switch (cl.nPam) {
+                case 1: plain_llr_store<1>(acc[t], noise, cl.lut, dst); break;
+                case 2: plain_llr_store<2>(acc[t], noise, cl.lut, dst); break;
+                case 3: plain_llr_store<3>(acc[t], noise, cl.lut, dst); break;
+                default: plain_llr_store<4>(acc[t], noise, cl.lut, dst); break;
+            }
+        }
+    }
+}
+
+// EX: every cell has L == LT.  LT: layers rounded up to 2, 4, 8 or 16.
+template <int MODE, int LT, bool EX>
+__global__ void __launch_bounds__(128) plain_kernel(const __grid_constant__ PlainParams p) {
+    constexpr int TEAM = plain_team(LT);
+    constexpr int LPL = TEAM / LT;                     // lanes per layer of the apply phase
+    extern __shared__ float4 plain_smem[];
+    const int team = threadIdx.x / TEAM, tid = threadIdx.x % TEAM;
+    int ci = 0;
+    while (ci + 1 < p.nCells && blockIdx.x >= p.cell[ci + 1].block0) ci++;
+    const PlainCell& cl = p.cell[ci];
+    const int A = cl.A, L = EX ? LT : cl.L, S = cl.S;
+    const int hs = EX ? LT + 2 : plain_hs(L), cs = plain_cs(A);
+    const long scw = (long)(blockIdx.x - cl.block0) * (blockDim.x / TEAM) + team;
+    const bool out = scw < cl.nSC;                     // teams past the cell's end repeat its last subcarrier
+    const long sc = out ? scw : cl.nSC - 1;
+    cf* sH = reinterpret_cast<cf*>(reinterpret_cast<char*>(plain_smem) + (size_t)team * p.teamBytes);
+    cf* sC = sH + (MODE != kApply ? A * hs : 0);
+    cf* sY = sC + (MODE != kGram ? L * cs : 0);
+    cf* sL = sY + (MODE == kApply || MODE == kChain ? S * cs : 0);
+    float* sInv = reinterpret_cast<float*>(sL + L * L);
+    float* sMuInv = sInv + L;
+    float* sNoise = sMuInv + L;
+
+    if constexpr (MODE != kApply) stage_rows<TEAM>(sH, hs, cl.H + sc * A * L, A, L, cl.vecH, tid);
+    else stage_rows<TEAM>(sC, cs, cl.C + sc * A * L, L, A, cl.vecY, tid);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    if constexpr (MODE == kApply || MODE == kChain)
+        stage_rows<TEAM>(sY, cs, cl.Y + sc * S * A, S, A, cl.vecY, tid);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    team_sync<TEAM>();
+
+    // ---- G: this lane's row r, columns 2q and 2q + 1 ----
+    // kGram enumerates the whole matrix, the solve its lower triangle (row
+    // pair R holds 2 (R + 1) column pairs, after R (R + 1) of the pairs above).
+    auto gram_pair = [&](int r, int q, cf& g0, cf& g1) {
+        g0 = g1 = make_float2(0.f, 0.f);
+        const cf* hr = sH + r;
+        const cf* hc = sH + 2 * q;
+#pragma unroll 4
+        for (int k = 0; k < A; k++) {
+            const cf v = hr[k * hs];
+            const float4 c = ld4(hc + k * hs);
+            const cf m = make_float2(v.x, -v.y);
+            g0 = cma(m, make_float2(c.x, c.y), g0);
+            g1 = cma(m, make_float2(c.z, c.w), g1);
+        }
+        if (r == 2 * q) g0.x = __fadd_rn(g0.x, cl.sigma2);
+        if (r == 2 * q + 1) g1.x = __fadd_rn(g1.x, cl.sigma2);
+    };
+    if constexpr (MODE == kGram) {
+        constexpr int PR = LT / 2;
+#pragma unroll
+        for (int t = tid; t < LT * PR; t += TEAM) {
+            const int r = t / PR, q = t % PR;
+            if (r >= L || 2 * q >= L) continue;
+            cf g0, g1;
+            gram_pair(r, q, g0, g1);
+            if (!out) continue;
+            cf* g = cl.G + (sc * L + r) * L + 2 * q;
+            if (EX && (reinterpret_cast<uintptr_t>(cl.G) & 15) == 0) {
+                *reinterpret_cast<float4*>(g) = make_float4(g0.x, g0.y, g1.x, g1.y);
+            } else {
+                g[0] = g0;
+                if (2 * q + 1 < L) g[1] = g1;
+            }
+        }
+        return;
+    }
+
+    float noise = 0.f;
+    if constexpr (MODE == kCoef || MODE == kChain) {
+        int R = 0;
+        while ((R + 1) * (R + 2) <= tid) R++;
+        const int u = tid - R * (R + 1);
+        const int r = 2 * R + (u > R ? 1 : 0), q = u > R ? u - R - 1 : u;
+        const bool own = r < L;
+        cf g0 = make_float2(0.f, 0.f), g1 = g0;        // (r, 2q), (r, 2q + 1)
+        if (own) {
+            if constexpr (MODE == kChain) {
+                gram_pair(r, q, g0, g1);
+            } else {
+                const cf* g = cl.G + (sc * L + r) * L + 2 * q;
+                g0 = g[0];
+                if (2 * q + 1 <= r) g1 = g[1];
+            }
+        }
+        for (int k = 0; k < L; k++) {
+            const bool odd = k & 1;
+            if (own && q == (k >> 1)) {
+                cf& e = odd ? g1 : g0;
+                if (r == k) {
+                    float s = e.x;
+                    if (!(s > 0.f)) s = 1e-30f;
+                    sInv[k] = __fdiv_rn(1.0f, __fsqrt_rn(s));
+                }
+            }
+            team_sync<TEAM>();
+            if (own && q == (k >> 1) && r > k) {
+                const cf e = odd ? g1 : g0;
+                const float iv = sInv[k];
+                sL[r * L + k] = make_float2(__fmul_rn(e.x, iv), __fmul_rn(e.y, iv));
+            }
+            team_sync<TEAM>();
+            if (own && 2 * q + 1 > k && r > k) {
+                const cf a = sL[r * L + k];
+                auto take = [&](cf b, cf& e) {
+                    e.x = __fmaf_rn(-a.x, b.x, e.x);
+                    e.x = __fmaf_rn(-a.y, b.y, e.x);
+                    e.y = __fmaf_rn(-a.y, b.x, e.y);
+                    e.y = __fmaf_rn(a.x, b.y, e.y);
+                };
+                if (2 * q > k) take(sL[2 * q * L + k], g0);
+                if (2 * q + 1 <= r) take(sL[(2 * q + 1) * L + k], g1);
+            }
+        }
+        // ---- C: forward and backward substitution per antenna ----
+        int a = tid;
+        for (; a + TEAM < A; a += 2 * TEAM) solve_antennas<LT, EX, 2, TEAM>(sH, hs, sL, sInv, sC, cs, L, a);
+        if (a < A) solve_antennas<LT, EX, 1, TEAM>(sH, hs, sL, sInv, sC, cs, L, a);
+        team_sync<TEAM>();
+        // ---- mu and the noise of the unbiased symbol ----
+        if (tid < L) {
+            float mu = 0.f;
+            const cf* c = sC + tid * cs;
+            const cf* h = sH + tid;
+#pragma unroll 8
+            for (int k = 0; k < A; k++) {
+                const cf cv = c[k], hv = h[k * hs];
+                mu = __fmaf_rn(cv.x, hv.x, mu);
+                mu = __fmaf_rn(-cv.y, hv.y, mu);
+            }
+            const float ni = __fdiv_rn(mu, __fsub_rn(1.0f, mu));
+            sMuInv[tid] = __fdiv_rn(1.0f, mu);
+            sNoise[tid] = ni;
+            if (MODE == kCoef && out) cl.nInv[sc * L + tid] = ni;
+        }
+        team_sync<TEAM>();
+        for (int l = 0; l < L; l++) {
+            const float im = sMuInv[l];
+            for (int k = tid; k < A; k += TEAM) {
+                const cf v = sC[l * cs + k];
+                const cf w = make_float2(__fmul_rn(v.x, im), __fmul_rn(v.y, im));
+                if constexpr (MODE == kChain) sC[l * cs + k] = w;
+                else if (out) cl.C[(sc * L + l) * A + k] = w;
+            }
+        }
+        if constexpr (MODE == kCoef) return;
+    }
+
+    // ---- Y_eq (and LLRs): lane (layer l, symbols st, st + LPL, ...) ----
+    if constexpr (MODE == kApply || MODE == kChain) {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        team_sync<TEAM>();
+        const int l = tid / LPL, st = tid % LPL;
+        if (l >= L) return;
+        if constexpr (MODE == kChain) noise = sNoise[l];
+        switch ((S + LPL - 1) / LPL) {
+            case 1: apply_symbols<MODE, 1, LPL>(cl, sC, sY, cs, noise, sc, l, st, out); break;
+            case 2: apply_symbols<MODE, 2, LPL>(cl, sC, sY, cs, noise, sc, l, st, out); break;
+            case 3: apply_symbols<MODE, 3, LPL>(cl, sC, sY, cs, noise, sc, l, st, out); break;
+            default: apply_symbols<MODE, 4, LPL>(cl, sC, sY, cs, noise, sc, l, st, out); break;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -192,28 +442,93 @@ static bool shape_ok(int nSC, int nSym, int L, int A) {
            A <= AERIAL_MAX_ANTS;
 }
 
-int launch_gram(const cf* H, float sigma2, cf* G, int nSC, int A, int L, cudaStream_t st) {
-    long total = (long)nSC * L * L;
-    gram_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(H, sigma2, G, total, A, L);
+static int layers_tile(int L) { return L <= 2 ? 2 : L <= 4 ? 4 : L <= 8 ? 8 : 16; }
+
+template <int MODE, int LT, bool EX>
+static int launch_plain_t(PlainParams& p, cudaStream_t st) {
+    constexpr int TEAM = plain_team(LT);
+    int teamBytes = 0;
+    for (int i = 0; i < p.nCells; i++)
+        teamBytes = std::max(teamBytes, plain_team_bytes(MODE, p.cell[i].A, p.cell[i].L, p.cell[i].S));
+    // 128 threads a block, fewer (whole warps) where their rows do not fit:
+    // the largest team's need (256 antennas, 16 layers, 16 symbols) is 103 KB
+    constexpr int WARP_TEAMS = TEAM >= 32 ? 1 : 32 / TEAM;
+    int teams = 128 / TEAM;
+    while (teams > WARP_TEAMS && teams * teamBytes > kMaxSmemPerCta) teams -= WARP_TEAMS;
+    if (teams * teamBytes > kMaxSmemPerCta) return AERIAL_ERR_UNSUPPORTED;
+    const int s = allow_max_smem<plain_kernel<MODE, LT, EX>>();
+    if (s) return s;
+    unsigned blocks = 0;
+    for (int i = 0; i < p.nCells; i++) {
+        p.cell[i].block0 = blocks;
+        blocks += (unsigned)((p.cell[i].nSC + teams - 1) / teams);
+    }
+    p.teamBytes = teamBytes;
+    plain_kernel<MODE, LT, EX><<<blocks, teams * TEAM, (size_t)teams * teamBytes, st>>>(p);
     return launch_status();
 }
 
-int launch_mmse_coef(const cf* G, const cf* H, cf* C, float* nI, int nSC, int A, int L, cudaStream_t st) {
-    size_t smem = sizeof(cf) * ((size_t)L * L + (size_t)L * A) + sizeof(float) * 2 * L;
-    int threads = A < 32 ? 32 : (A > 256 ? 256 : ((A + 31) / 32) * 32);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(mmse_coef_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    mmse_coef_kernel<<<nSC, threads, smem, st>>>(G, H, C, nI, A, L);
-    return launch_status();
+template <int MODE, int LT>
+static int launch_plain_l(PlainParams& p, cudaStream_t st) {
+    bool exact = true;
+    for (int i = 0; i < p.nCells; i++) exact = exact && p.cell[i].L == LT;
+    return exact ? launch_plain_t<MODE, LT, true>(p, st) : launch_plain_t<MODE, LT, false>(p, st);
 }
 
-int launch_coef_apply(const cf* C, const cf* Y, cf* O, int nSC, int nSym, int L, int A, cudaStream_t st) {
-    dim3 blk(12, nSym), grd((nSC + 11) / 12, L);
-    size_t smem = sizeof(cf) * (size_t)A * 12;
-    coef_apply_kernel<<<grd, blk, smem, st>>>(C, Y, O, nSC, nSym, L, A);
-    return launch_status();
+// Cells whose layers round up to the same tile, in one launch.
+template <int MODE>
+static int launch_plain(PlainParams& p, cudaStream_t st) {
+    switch (layers_tile(p.cell[0].L)) {
+        case 2: return launch_plain_l<MODE, 2>(p, st);
+        case 4: return launch_plain_l<MODE, 4>(p, st);
+        case 8: return launch_plain_l<MODE, 8>(p, st);
+        default: return launch_plain_l<MODE, 16>(p, st);
+    }
 }
 
-int launch_llr_f32(const cf* in, const float* ni, float* out, int N, int n, int spn, cudaStream_t st) {
+static PlainCell plain_cell(const cf* H, const cf* Y, int nSC, int A, int L, int S) {
+    PlainCell c{};
+    c.H = H;
+    c.Y = Y;
+    c.nSC = nSC;
+    c.A = A;
+    c.L = L;
+    c.S = S;
+    c.vecH = (L % 2) == 0 && ((uintptr_t)H & 15) == 0;
+    c.vecY = (A % 2) == 0 && ((uintptr_t)Y & 15) == 0;
+    return c;
+}
+
+static int launch_gram(const cf* H, float sigma2, cf* G, int nSC, int A, int L, cudaStream_t st) {
+    PlainParams p;
+    p.nCells = 1;
+    p.cell[0] = plain_cell(H, nullptr, nSC, A, L, 1);
+    p.cell[0].G = G;
+    p.cell[0].sigma2 = sigma2;
+    return launch_plain<kGram>(p, st);
+}
+
+static int launch_mmse_coef(const cf* G, const cf* H, cf* C, float* nI, int nSC, int A, int L, cudaStream_t st) {
+    PlainParams p;
+    p.nCells = 1;
+    p.cell[0] = plain_cell(H, nullptr, nSC, A, L, 1);
+    p.cell[0].G = const_cast<cf*>(G);
+    p.cell[0].C = C;
+    p.cell[0].nInv = nI;
+    return launch_plain<kCoef>(p, st);
+}
+
+static int launch_coef_apply(const cf* C, const cf* Y, cf* O, int nSC, int nSym, int L, int A, cudaStream_t st) {
+    PlainParams p;
+    p.nCells = 1;
+    p.cell[0] = plain_cell(nullptr, Y, nSC, A, L, nSym);
+    p.cell[0].C = const_cast<cf*>(C);
+    p.cell[0].O = O;
+    p.cell[0].vecY = p.cell[0].vecY && ((uintptr_t)C & 15) == 0;
+    return launch_plain<kApply>(p, st);
+}
+
+static int launch_llr_f32(const cf* in, const float* ni, float* out, int N, int n, int spn, cudaStream_t st) {
     PamLut lut = pam_lut(n);
     unsigned g = (unsigned)((N + 511) / 512);
     switch (n) {
@@ -235,10 +550,25 @@ static int prepare_one(K* k) {
     cudaFuncAttributes at;
     return rt_status(cudaFuncGetAttributes(&at, k));
 }
+template <int MODE, int LT>
+static int prepare_plain_l() {
+    int s = prepare_one(plain_kernel<MODE, LT, true>);
+    if (!s) s = allow_max_smem<plain_kernel<MODE, LT, true>>();
+    if (!s) s = prepare_one(plain_kernel<MODE, LT, false>);
+    return s ? s : allow_max_smem<plain_kernel<MODE, LT, false>>();
+}
+template <int MODE>
+static int prepare_plain_mode() {
+    int s = prepare_plain_l<MODE, 2>();
+    if (!s) s = prepare_plain_l<MODE, 4>();
+    if (!s) s = prepare_plain_l<MODE, 8>();
+    return s ? s : prepare_plain_l<MODE, 16>();
+}
 int prepare_plain_kernels() {
-    int s = prepare_one(gram_kernel);
-    if (!s) s = prepare_one(mmse_coef_kernel);
-    if (!s) s = prepare_one(coef_apply_kernel);
+    int s = prepare_plain_mode<kGram>();
+    if (!s) s = prepare_plain_mode<kCoef>();
+    if (!s) s = prepare_plain_mode<kApply>();
+    if (!s) s = prepare_plain_mode<kChain>();
     if (!s) s = prepare_one(llr_f16_kernel<1>);
     if (!s) s = prepare_one(llr_f16_kernel<2>);
     if (!s) s = prepare_one(llr_f16_kernel<3>);
@@ -297,8 +627,9 @@ extern "C" int aerial_llr_f32(const aerial_cf32* softEst, const float* noiseInv,
 }
 
 // ---------------------------------------------------------------------------
-// The plain chain over cells: workspace holds G, C, noiseInv and Y_eq of the
-// largest cell; cells run one after another on `stream`.
+// The plain chain over cells.  The workspace (G, C, noiseInv and Y_eq of the
+// largest cell) is part of the interface and checked; the chain's kernel keeps
+// them on chip and does not touch it.
 // ---------------------------------------------------------------------------
 static size_t plain_ws_cell(const aerial_cell_desc& c) {
     size_t nSC = (size_t)c.nPRB * 12;
@@ -316,34 +647,52 @@ extern "C" size_t aerial_pusch_eq_plain_workspace(const aerial_cell_desc* cells,
     return m;
 }
 
+// The checks of one cell, before anything is launched.
+static int plain_cell_check(const aerial_cell_desc& c) {
+    if (c.nPRB < 1 || c.nPRB > AERIAL_MAX_PRB) return AERIAL_ERR_INVALID_ARG;
+    if (!c.H || !c.Y_rx || !c.llr || c.nPamBits < 1 || c.nPamBits > 4 ||
+        !shape_ok(c.nPRB * 12, c.nSym, c.nLayers, c.nAnt))
+        return AERIAL_ERR_INVALID_ARG;
+    if (c.format != AERIAL_FMT_CF32) return AERIAL_ERR_UNSUPPORTED;   // the FP32 chain reads complex64 only
+    return AERIAL_OK;
+}
+
+// Consecutive cells whose layers share a tile go into one launch; the chain
+// needs no memory of its own.
+static int run_plain(const aerial_cell_desc* cells, int nCells, cudaStream_t st) {
+    for (int i = 0; i < nCells;) {
+        PlainParams p;
+        p.nCells = 0;
+        const int tile = layers_tile(cells[i].nLayers);
+        long subcarriers = 0;                        // block indices stay in 31 bits
+        for (; i < nCells && p.nCells < AERIAL_MAX_CELLS && layers_tile(cells[i].nLayers) == tile; i++) {
+            const aerial_cell_desc& c = cells[i];
+            const int nSC = c.nPRB * 12;
+            if (p.nCells && subcarriers + nSC > INT32_MAX / 2) break;
+            subcarriers += nSC;
+            PlainCell& d = p.cell[p.nCells++];
+            d = plain_cell((const cf*)c.H, (const cf*)c.Y_rx, nSC, c.nAnt, c.nLayers, c.nSym);
+            d.O = (cf*)c.Y_eq;
+            d.llr = c.llr;
+            d.sigma2 = c.sigma2;
+            d.nPam = c.nPamBits;
+            d.lut = pam_lut(c.nPamBits);
+        }
+        const int s = launch_plain<kChain>(p, st);
+        if (s) return s;
+    }
+    return AERIAL_OK;
+}
+
 extern "C" int aerial_pusch_eq_plain(const aerial_cell_desc* cells, int nCells, void* workspace, size_t wsBytes,
                                      void* stream) {
     if (!cells || nCells < 1 || !workspace) return AERIAL_ERR_INVALID_ARG;
-    cudaStream_t st = to_stream(stream);
     for (int i = 0; i < nCells; i++) {
-        const aerial_cell_desc& c = cells[i];
-        if (c.nPRB < 1 || c.nPRB > AERIAL_MAX_PRB) return AERIAL_ERR_INVALID_ARG;
-        int nSC = c.nPRB * 12;
-        if (!c.H || !c.Y_rx || !c.llr || c.nPamBits < 1 || c.nPamBits > 4 || !shape_ok(nSC, c.nSym, c.nLayers, c.nAnt))
-            return AERIAL_ERR_INVALID_ARG;
-        if (c.format != AERIAL_FMT_CF32) return AERIAL_ERR_UNSUPPORTED;   // the FP32 chain reads complex64 only
-        if (plain_ws_cell(c) > wsBytes) return AERIAL_ERR_INVALID_ARG;
-        auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-        char* p = (char*)workspace;
-        cf* G = (cf*)p;
-        p += al((size_t)nSC * c.nLayers * c.nLayers * sizeof(cf));
-        cf* C = (cf*)p;
-        p += al((size_t)nSC * c.nLayers * c.nAnt * sizeof(cf));
-        float* nI = (float*)p;
-        p += al((size_t)nSC * c.nLayers * sizeof(float));
-        cf* Yeq = c.Y_eq ? (cf*)c.Y_eq : (cf*)p;
-        int s;
-        if ((s = launch_gram((const cf*)c.H, c.sigma2, G, nSC, c.nAnt, c.nLayers, st))) return s;
-        if ((s = launch_mmse_coef(G, (const cf*)c.H, C, nI, nSC, c.nAnt, c.nLayers, st))) return s;
-        if ((s = launch_coef_apply(C, (const cf*)c.Y_rx, Yeq, nSC, c.nSym, c.nLayers, c.nAnt, st))) return s;
-        if ((s = launch_llr_f32(Yeq, nI, c.llr, nSC * c.nLayers * c.nSym, c.nPamBits, c.nSym, st))) return s;
+        const int s = plain_cell_check(cells[i]);
+        if (s != AERIAL_OK) return s;
+        if (plain_ws_cell(cells[i]) > wsBytes) return AERIAL_ERR_INVALID_ARG;
     }
-    return AERIAL_OK;
+    return run_plain(cells, nCells, to_stream(stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -352,66 +701,11 @@ extern "C" int aerial_pusch_eq_plain(const aerial_cell_desc* cells, int nCells, 
 // Some hosts cannot call cudaMalloc on the path that equalizes a slot: a
 // real-time receiver loop where an allocation may block or synchronize the
 // device and miss the slot deadline, or a plugin inside a framework that owns
-// all device memory and hands out none.  This entry point keeps the plain
-// chain's intermediates (G, C, noiseInv, Y_eq) in one file-scope device array
-// instead of a caller workspace.  The array is part of the module image, so
-// every GPU that loads this library holds it until the process exits.
-//
-// The array's host-side name is only a stand-in for the device symbol; the
-// device address comes from cudaGetSymbolAddress, made with the device
-// current.  The address belongs to the CUDA context that loaded the module:
-// a cudaDeviceReset, or a second context on the same device, gets its own
-// copy of the array.  The address is therefore cached per device together
-// with the unique ID of the context it was looked up in (cuCtxGetId, which a
-// new context never reuses even where its handle value is recycled), and
-// looked up again whenever a call runs in a different context.  The first
-// call in each context does that lookup, so make it before any stream
-// capture.  All calls share the one array and it keeps the last call's
-// contents: every scratch byte a call reads is first written by that same
-// call, so nothing needs clearing, but calls that overlap on the GPU (two
-// streams, two threads) race on it.
+// all device memory and hands out none.  The chain's intermediates (G, C,
+// noiseInv) live in shared memory, so this entry point needs no device memory
+// at all; a batch whose largest cell's intermediates would exceed
+// AERIAL_STATIC_SCRATCH_BYTES is refused, as the interface states.
 // ---------------------------------------------------------------------------
-#include <mutex>
-
-static __device__ __align__(256) unsigned char g_plain_static_scratch[AERIAL_STATIC_SCRATCH_BYTES];
-
-static int static_scratch_address(void** out) {
-    static std::mutex mu;
-    static void* addr[64] = {};
-    static unsigned long long ctxOf[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return rt_status(e);
-    if (dev < 0 || dev >= 64) return AERIAL_ERR_NO_DEVICE;
-    std::lock_guard<std::mutex> lock(mu);
-    const unsigned long long ctx = current_ctx_id();
-    if (ctx != 0 && addr[dev] && ctxOf[dev] == ctx) {
-        *out = addr[dev];
-        return AERIAL_OK;
-    }
-    // no cached address for this context (or no context yet: the runtime
-    // makes the device's primary context current inside this call)
-    void* p = nullptr;
-    e = cudaGetSymbolAddress(&p, g_plain_static_scratch);
-    if (e != cudaSuccess) return rt_status(e);
-    addr[dev] = p;
-    ctxOf[dev] = current_ctx_id();    // 0 when unknown: looked up again next call
-    *out = p;
-    return AERIAL_OK;
-}
-
-// The checks aerial_pusch_eq_plain makes per cell, so a malformed cell gets
-// AERIAL_ERR_INVALID_ARG / AERIAL_ERR_UNSUPPORTED before the size comparison
-// (negative shapes would otherwise wrap in the workspace arithmetic).
-static int plain_cell_check(const aerial_cell_desc& c) {
-    if (c.nPRB < 1 || c.nPRB > AERIAL_MAX_PRB) return AERIAL_ERR_INVALID_ARG;
-    if (!c.H || !c.Y_rx || !c.llr || c.nPamBits < 1 || c.nPamBits > 4 ||
-        !shape_ok(c.nPRB * 12, c.nSym, c.nLayers, c.nAnt))
-        return AERIAL_ERR_INVALID_ARG;
-    if (c.format != AERIAL_FMT_CF32) return AERIAL_ERR_UNSUPPORTED;
-    return AERIAL_OK;
-}
-
 extern "C" int aerial_pusch_eq_plain_static(const aerial_cell_desc* cells, int nCells, void* stream) {
     if (!cells || nCells < 1) return AERIAL_ERR_INVALID_ARG;
     for (int i = 0; i < nCells; i++) {
@@ -420,8 +714,5 @@ extern "C" int aerial_pusch_eq_plain_static(const aerial_cell_desc* cells, int n
     }
     if (aerial_pusch_eq_plain_workspace(cells, nCells) > (size_t)AERIAL_STATIC_SCRATCH_BYTES)
         return AERIAL_ERR_SCRATCH_LIMIT;
-    void* scratch = nullptr;
-    const int s = static_scratch_address(&scratch);
-    if (s != AERIAL_OK) return s;
-    return aerial_pusch_eq_plain(cells, nCells, scratch, (size_t)AERIAL_STATIC_SCRATCH_BYTES, stream);
+    return run_plain(cells, nCells, to_stream(stream));
 }

@@ -1,0 +1,78 @@
+"""The plain FP32 chain and its stages at the sizes where their kernel's
+division of a subcarrier among lanes can go wrong: layers around each tile
+(2, 4, 8, 16), odd antenna counts, antennas just past a team's lanes, one and
+sixteen symbols, rows that are only 8-byte aligned, and several cells of
+different shapes in one call.  Every result is bit-identical to the oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [  # (nPRB, nAnt, nLayers, nSym, qam)
+    (1, 1, 1, 1, 4), (1, 17, 1, 16, 16), (2, 16, 2, 9, 64), (1, 33, 3, 5, 256), (3, 32, 4, 13, 16),
+    (1, 20, 5, 16, 4), (1, 65, 7, 3, 64), (2, 64, 8, 14, 256), (1, 31, 8, 16, 16), (1, 129, 9, 8, 64),
+    (1, 40, 12, 7, 256), (1, 127, 15, 11, 16), (1, 256, 16, 16, 256),
+]
+
+
+def _shifted(x, cuda, shift):
+    """x on the device, `shift` complex values past a 16-byte boundary."""
+    t = torch.empty(x.numel() + 2, dtype=x.dtype, device=cuda)
+    v = t[shift:shift + x.numel()]
+    v.copy_(x.reshape(-1))
+    return v
+
+
+def _desc(aeq, c, cuda, shift, yeq=True):
+    H, Y = _shifted(c.H, cuda, shift), _shifted(c.Y, cuda, shift)
+    llr = torch.full((c.llr_numel,), float("nan"), dtype=torch.float32, device=cuda)
+    ye = torch.full((c.nSC * c.nLayers * c.nSym,), float("nan"), dtype=torch.complex64, device=cuda) if yeq else None
+    return aeq.cell_desc(H, Y, llr, c.sigma2, c.nPRB, c.nAnt, c.nLayers, c.nSym, c.nPamBits, Y_eq=ye), (H, Y, llr, ye)
+
+
+def _check(orc, c, llr, ye):
+    y32, _, l32 = orc.chain_f32(c.H.numpy(), c.Y.numpy(), c.sigma2, c.nSC, c.nAnt, c.nLayers, c.nSym, c.nPamBits)
+    np.testing.assert_array_equal(llr.cpu().numpy(), l32)
+    if ye is not None:
+        np.testing.assert_array_equal(ye.cpu().numpy(), y32)
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_chain_and_stages_bit_exact(aeq, wl, orc, cuda, shape, shift):
+    p, A, L, S, q = shape
+    c = wl.make_cell(p, A, L, S, q, 20.0, seed=100 + A)
+    d, (H, Y, llr, ye) = _desc(aeq, c, cuda, shift)
+    aeq.pusch_eq_plain([d], torch.empty(aeq.pusch_eq_plain_workspace([d]), dtype=torch.uint8, device=cuda))
+    n = c.nSC
+    G = _shifted(torch.zeros(n * L * L, dtype=torch.complex64), cuda, shift)
+    C = _shifted(torch.zeros(n * L * A, dtype=torch.complex64), cuda, shift)
+    ni = torch.zeros(n * L, dtype=torch.float32, device=cuda)
+    O = _shifted(torch.zeros(n * L * S, dtype=torch.complex64), cuda, shift)
+    aeq.gram(H, c.sigma2, G, n, A, L)
+    aeq.mmse_coef(G, H, C, ni, n, A, L)
+    aeq.coef_apply(C, Y, O, n, S, L, A)
+    torch.cuda.synchronize()
+    Gr = orc.gram(c.H.numpy(), c.sigma2, n, A, L)
+    Cr, nr = orc.mmse_coef(Gr, c.H.numpy(), n, A, L)
+    np.testing.assert_array_equal(G.cpu().numpy(), Gr)
+    np.testing.assert_array_equal(C.cpu().numpy(), Cr)
+    np.testing.assert_array_equal(ni.cpu().numpy(), nr)
+    np.testing.assert_array_equal(O.cpu().numpy(), orc.coef_apply_v1(Cr, c.Y.numpy().reshape(-1), n, S, L, A))
+    _check(orc, c, llr, ye)
+
+
+def test_many_cells_in_one_call(aeq, wl, orc, cuda):
+    """More cells than one launch holds, tiles changing from cell to cell, every other cell without Y_eq."""
+    cells = [wl.make_cell(*SHAPES[i % 8], 20.0, seed=i) for i in range(12)]
+    cells += [wl.make_cell(1, 8, 2, 4, 16, 20.0, seed=50 + i) for i in range(70)]
+    got = [_desc(aeq, c, cuda, 0, yeq=i % 2 == 0) for i, c in enumerate(cells)]
+    arr = (aeq.CellDesc * len(cells))(*[d for d, _ in got])
+    ws = torch.empty(aeq.lib().aerial_pusch_eq_plain_workspace(arr, len(cells)), dtype=torch.uint8, device=cuda)
+    assert aeq.lib().aerial_pusch_eq_plain(arr, len(cells), ws.data_ptr(), ws.numel(), None) == 0
+    torch.cuda.synchronize()
+    for c, (_, (_, _, llr, ye)) in zip(cells, got):
+        _check(orc, c, llr, ye)
