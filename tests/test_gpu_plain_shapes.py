@@ -18,6 +18,10 @@ SHAPES = [  # (nPRB, nAnt, nLayers, nSym, qam)
 ]
 
 
+def _d(x, dev):
+    return torch.from_numpy(np.ascontiguousarray(x)).to(dev)
+
+
 def _shifted(x, cuda, shift):
     """x on the device, `shift` complex values past a 16-byte boundary."""
     t = torch.empty(x.numel() + 2, dtype=x.dtype, device=cuda)
@@ -76,3 +80,21 @@ def test_many_cells_in_one_call(aeq, wl, orc, cuda):
     torch.cuda.synchronize()
     for c, (_, (_, _, llr, ye)) in zip(cells, got):
         _check(orc, c, llr, ye)
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (13, 8, 8, 8), (24, 31, 9, 9), (12, 32, 16, 16), (12, 40, 8, 14),
+                                   (12, 65, 3, 11), (12, 256, 16, 7)])
+def test_coef_apply_tc_sizes(aeq, orc, cuda, shape, shift):
+    """Tiles with missing layers and symbols, antenna counts around the groups of four k-steps (32 antennas)."""
+    nSC, A, L, S = shape
+    v = orc.ref_uniform(7, nSC * L * A * 2 + nSC * S * A * 2, 1.0)
+    C = v[: nSC * L * A * 2].view(np.complex64)
+    Y = v[nSC * L * A * 2:].view(np.complex64)
+    O = torch.zeros(nSC * L * S, dtype=torch.complex64, device=cuda)
+    aeq.coef_apply_tc(_shifted(torch.from_numpy(C.copy()), cuda, shift), _shifted(torch.from_numpy(Y.copy()), cuda, shift),
+                      O, nSC, S, L, A)
+    torch.cuda.synchronize()
+    ref = orc.coef_apply_v2_model(C, Y, nSC, S, L, A)
+    # both sum the same exact FP16 products in FP32, in another order: A complex products of size <= 1/2 each
+    np.testing.assert_allclose(O.cpu().numpy(), ref, rtol=0, atol=2 * A * 2.0 ** -23 * max(1.0, A / 8))
