@@ -404,34 +404,122 @@ __global__ void __launch_bounds__(128) plain_kernel(const __grid_constant__ Plai
 }
 
 // ---------------------------------------------------------------------------
-// LLR demapper: one thread per symbol (llr_v1_baseline / llr_v3 shape).
+// LLR demapper: one thread per symbol (llr_v1_baseline / llr_v3 shape).  It is
+// bound by its writes, 2 N values per symbol read: a thread's LLRs go out in
+// one store as wide as they are (32 bytes of 256-QAM in FP32 fill a sector;
+// as four 8-byte stores each of a warp's requests left every sector of 1 KB a
+// quarter full).  14-symbol 256-QAM of 8 slots of 1,584 subcarriers x 8
+// layers, 57 MB: 21.5 -> 12 us.  64-QAM rows (24 bytes) cross through shared
+// memory into 16-byte stores.  Less aligned outputs take the narrow stores.
 // ---------------------------------------------------------------------------
-template <int N>
-__global__ void __launch_bounds__(512) llr_f16_kernel(const __half2* __restrict__ in,
-                                                       const float* __restrict__ ni,
-                                                       __half* __restrict__ out, int count, PamLut lut) {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= count) return;
-    __half2 v = in[idx];
-    float o[2 * N];
-    pam_llr<N>(__low2float(v), __high2float(v), ni[idx], lut, o);
-    __half* dst = out + (long)idx * 2 * N;
+constexpr int kLlrThreads = 512;
+constexpr int kLlrPerThread = 2;               // symbols a thread loads before it demaps the first
+
+// W: 4-byte words of LLRs per symbol.
+template <int W>
+__device__ __forceinline__ void store_words(uint32_t* dst, const uint32_t (&v)[W]) {
+    if constexpr (W == 8)
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(dst), "r"(v[0]), "r"(v[1]),
+                     "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                     : "memory");
+    else if constexpr (W == 4)
+        *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+    else if constexpr (W == 2)
+        *reinterpret_cast<uint2*>(dst) = make_uint2(v[0], v[1]);
+    else
+        *dst = v[0];
+}
+
+// The block's symbols base .. base + 511 (count in all).  wide: out is aligned
+// to the row's store (16 bytes for rows of 3 or 6 words); otherwise NARROW
+// words at a time (FP32 LLR rows are 8-byte aligned, FP16 ones 4-byte).
+template <int W, int NARROW>
+__device__ __forceinline__ void write_rows(uint32_t* out, long base, int count, const uint32_t (&v)[W], bool wide) {
+    const long idx = base + threadIdx.x;
+    if constexpr (W == 6 || W == 3) {
+        __shared__ __align__(16) uint32_t rows[kLlrThreads * W];
+        if (wide && base + kLlrThreads <= count) {
 #pragma unroll
-    for (int j = 0; j < 2 * N; j += 2) *reinterpret_cast<__half2*>(dst + j) = __floats2half2_rn(o[j], o[j + 1]);
+            for (int j = 0; j < W; j++) rows[threadIdx.x * W + j] = v[j];
+            __syncthreads();
+            for (int e = threadIdx.x; e < kLlrThreads * W / 4; e += kLlrThreads)
+                reinterpret_cast<uint4*>(out + base * W)[e] = reinterpret_cast<const uint4*>(rows)[e];
+            __syncthreads();
+            return;
+        }
+    } else if (wide) {
+        if (idx < count) store_words<W>(out + idx * W, v);
+        return;
+    }
+    if (idx >= count) return;
+#pragma unroll
+    for (int j = 0; j < W; j += NARROW) {
+        uint32_t part[NARROW];
+#pragma unroll
+        for (int i = 0; i < NARROW; i++) part[i] = v[j + i];
+        store_words<NARROW>(out + idx * W + j, part);
+    }
 }
 
 template <int N>
-__global__ void __launch_bounds__(512) llr_f32_kernel(const cf* __restrict__ in, const float* __restrict__ ni,
-                                                       float* __restrict__ out, int count, int symsPerNoise,
-                                                       PamLut lut) {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= count) return;
-    cf v = in[idx];
-    float o[2 * N];
-    pam_llr<N>(v.x, v.y, ni[idx / symsPerNoise], lut, o);
-    float* dst = out + (long)idx * 2 * N;
+__global__ void __launch_bounds__(kLlrThreads) llr_f16_kernel(const __half2* __restrict__ in,
+                                                               const float* __restrict__ ni,
+                                                               __half* __restrict__ out, int count, bool wide,
+                                                               PamLut lut) {
+    __half2 v[kLlrPerThread];
+    float nv[kLlrPerThread];
+    const long base = (long)blockIdx.x * kLlrThreads * kLlrPerThread;
 #pragma unroll
-    for (int j = 0; j < 2 * N; j += 2) *reinterpret_cast<float2*>(dst + j) = make_float2(o[j], o[j + 1]);
+    for (int u = 0; u < kLlrPerThread; u++) {
+        const long at = min(base + u * kLlrThreads + (long)threadIdx.x, (long)count - 1);
+        v[u] = in[at];
+        nv[u] = ni[at];
+    }
+#pragma unroll
+    for (int u = 0; u < kLlrPerThread; u++) {
+        float o[2 * N];
+        pam_llr<N>(__low2float(v[u]), __high2float(v[u]), nv[u], lut, o);
+        uint32_t w[N];
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+            const __half2 h = __floats2half2_rn(o[2 * j], o[2 * j + 1]);
+            w[j] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        write_rows<N, 1>(reinterpret_cast<uint32_t*>(out), base + u * kLlrThreads, count, w, wide);
+    }
+}
+
+// noiseInv index = symbol / symsPerNoise: the block's first quotient by one
+// division, the rest from it (rcp = floor(2^32 / symsPerNoise) + 1, exact
+// while symsPerNoise <= 1024; a larger count changes at most once in a block).
+template <int N>
+__global__ void __launch_bounds__(kLlrThreads) llr_f32_kernel(const cf* __restrict__ in,
+                                                               const float* __restrict__ ni,
+                                                               float* __restrict__ out, int count, int symsPerNoise,
+                                                               unsigned rcp, bool wide, PamLut lut) {
+    cf v[kLlrPerThread];
+    float nv[kLlrPerThread];
+    const long base = (long)blockIdx.x * kLlrThreads * kLlrPerThread;
+    const int q0 = (int)(base / symsPerNoise);
+#pragma unroll
+    for (int u = 0; u < kLlrPerThread; u++) {
+        const long at = min(base + u * kLlrThreads + (long)threadIdx.x, (long)count - 1);
+        const unsigned r = (unsigned)(at - (long)q0 * symsPerNoise);
+        const int q = q0 + (symsPerNoise == 1 ? (int)r
+                            : symsPerNoise <= 1024 ? (int)__umulhi(r, rcp)
+                                                   : (r >= (unsigned)symsPerNoise ? 1 : 0));
+        v[u] = in[at];
+        nv[u] = ni[q];
+    }
+#pragma unroll
+    for (int u = 0; u < kLlrPerThread; u++) {
+        float o[2 * N];
+        pam_llr<N>(v[u].x, v[u].y, nv[u], lut, o);
+        uint32_t w[2 * N];
+#pragma unroll
+        for (int j = 0; j < 2 * N; j++) w[j] = __float_as_uint(o[j]);
+        write_rows<2 * N, 2>(reinterpret_cast<uint32_t*>(out), base + u * kLlrThreads, count, w, wide);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -528,14 +616,22 @@ static int launch_coef_apply(const cf* C, const cf* Y, cf* O, int nSC, int nSym,
     return launch_plain<kApply>(p, st);
 }
 
+// Whether rows of `words` 4-byte LLR words may be stored whole (write_rows).
+static bool llr_wide(const void* out, int words) {
+    const uintptr_t need = words == 6 || words == 3 ? 16 : 4 * (uintptr_t)words;
+    return ((uintptr_t)out & (need - 1)) == 0;
+}
+
 static int launch_llr_f32(const cf* in, const float* ni, float* out, int N, int n, int spn, cudaStream_t st) {
-    PamLut lut = pam_lut(n);
-    unsigned g = (unsigned)((N + 511) / 512);
+    const PamLut lut = pam_lut(n);
+    const unsigned g = ((unsigned)N + kLlrThreads * kLlrPerThread - 1) / (kLlrThreads * kLlrPerThread);
+    const unsigned rcp = spn > 1 ? (unsigned)(0x100000000ull / (unsigned)spn) + 1u : 0u;
+    const bool w = llr_wide(out, 2 * n);
     switch (n) {
-        case 1: llr_f32_kernel<1><<<g, 512, 0, st>>>(in, ni, out, N, spn, lut); break;
-        case 2: llr_f32_kernel<2><<<g, 512, 0, st>>>(in, ni, out, N, spn, lut); break;
-        case 3: llr_f32_kernel<3><<<g, 512, 0, st>>>(in, ni, out, N, spn, lut); break;
-        default: llr_f32_kernel<4><<<g, 512, 0, st>>>(in, ni, out, N, spn, lut); break;
+        case 1: llr_f32_kernel<1><<<g, kLlrThreads, 0, st>>>(in, ni, out, N, spn, rcp, w, lut); break;
+        case 2: llr_f32_kernel<2><<<g, kLlrThreads, 0, st>>>(in, ni, out, N, spn, rcp, w, lut); break;
+        case 3: llr_f32_kernel<3><<<g, kLlrThreads, 0, st>>>(in, ni, out, N, spn, rcp, w, lut); break;
+        default: llr_f32_kernel<4><<<g, kLlrThreads, 0, st>>>(in, ni, out, N, spn, rcp, w, lut); break;
     }
     return launch_status();
 }
@@ -605,16 +701,17 @@ extern "C" int aerial_coef_apply(const aerial_cf32* C, const aerial_cf32* Y_rx, 
 extern "C" int aerial_llr(const aerial_ch2* softEst, const float* noiseInv, uint16_t* llrOut, int N, int nPamBits,
                           void* stream) {
     if (!softEst || !noiseInv || !llrOut || N < 1 || nPamBits < 1 || nPamBits > 4) return AERIAL_ERR_INVALID_ARG;
-    PamLut lut = pam_lut(nPamBits);
-    unsigned g = (unsigned)((N + 511) / 512);
+    const PamLut lut = pam_lut(nPamBits);
+    const unsigned g = ((unsigned)N + kLlrThreads * kLlrPerThread - 1) / (kLlrThreads * kLlrPerThread);
     cudaStream_t st = to_stream(stream);
     const __half2* in = (const __half2*)softEst;
     __half* out = (__half*)llrOut;
+    const bool w = llr_wide(out, nPamBits);
     switch (nPamBits) {
-        case 1: llr_f16_kernel<1><<<g, 512, 0, st>>>(in, noiseInv, out, N, lut); break;
-        case 2: llr_f16_kernel<2><<<g, 512, 0, st>>>(in, noiseInv, out, N, lut); break;
-        case 3: llr_f16_kernel<3><<<g, 512, 0, st>>>(in, noiseInv, out, N, lut); break;
-        default: llr_f16_kernel<4><<<g, 512, 0, st>>>(in, noiseInv, out, N, lut); break;
+        case 1: llr_f16_kernel<1><<<g, kLlrThreads, 0, st>>>(in, noiseInv, out, N, w, lut); break;
+        case 2: llr_f16_kernel<2><<<g, kLlrThreads, 0, st>>>(in, noiseInv, out, N, w, lut); break;
+        case 3: llr_f16_kernel<3><<<g, kLlrThreads, 0, st>>>(in, noiseInv, out, N, w, lut); break;
+        default: llr_f16_kernel<4><<<g, kLlrThreads, 0, st>>>(in, noiseInv, out, N, w, lut); break;
     }
     return launch_status();
 }

@@ -82,6 +82,28 @@ def test_many_cells_in_one_call(aeq, wl, orc, cuda):
         _check(orc, c, llr, ye)
 
 
+@pytest.mark.parametrize("n", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,spn,shift", [(1, 1, 0), (511, 11, 0), (513, 1, 0), (5000, 1023, 0), (5000, 1024, 0),
+                                         (5000, 1025, 0), (4096, 7, 2), (1025, 14, 4)])
+def test_llr_sizes_bit_exact(aeq, orc, cuda, n, N, spn, shift):
+    """Partial blocks, symbols per noise value around the fast quotient's limit, outputs off the wide alignment."""
+    rng = np.random.default_rng(N + n)
+    soft = (rng.standard_normal(2 * N) * 0.7).astype(np.float32)
+    ni = (10 ** rng.uniform(0, 3, N // spn + 1)).astype(np.float32)
+    buf = torch.full((N * 2 * n + 16,), float("nan"), dtype=torch.float32, device=cuda)
+    out = buf[shift:shift + N * 2 * n]
+    aeq.llr_f32(_d(soft, cuda), _d(ni, cuda), out, N, n, spn)
+    s16, ni1 = orc.ref_llr_inputs(N, N)
+    buf16 = torch.full((N * 2 * n + 16,), -1, dtype=torch.int16, device=cuda)
+    out16 = buf16[shift:shift + N * 2 * n]
+    aeq.llr(_d(s16.view(np.int16), cuda), _d(ni1, cuda), out16, N, n)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy(), orc.llr_f32(soft.view(np.complex64), ni, n, spn))
+    np.testing.assert_array_equal(out16.cpu().numpy().view(np.uint16), orc.llr_f16io(s16, ni1, n))
+    assert torch.isnan(buf[:shift]).all() and torch.isnan(buf[shift + N * 2 * n:]).all()     # nothing else written
+    assert (buf16[:shift] == -1).all() and (buf16[shift + N * 2 * n:] == -1).all()
+
+
 @pytest.mark.parametrize("shift", [0, 1])
 @pytest.mark.parametrize("shape", [(1, 1, 1, 1), (13, 8, 8, 8), (24, 31, 9, 9), (12, 32, 16, 16), (12, 40, 8, 14),
                                    (12, 65, 3, 11), (12, 256, 16, 7)])
