@@ -10,11 +10,10 @@
 namespace aeq {
 
 // ---------------------------------------------------------------------------
-// One kernel for every stage but the stand-alone demapper.  A team of TEAM
+// One kernel for the solve, the apply and the whole chain.  A team of TEAM
 // lanes owns a subcarrier; its H, Y and C sit in shared memory, G and the
 // trailing block of the factor in registers.
 //
-//   kGram   H -> G                       gram_scalar (src/aerial_bottleneck.cu:56-80), M = H^H
 //   kCoef   G, H -> C, noiseInv          the FP32 Cholesky MMSE solve
 //   kApply  C, Y -> Y_eq                 coef_apply_v1_scalar (src/aerial_coef_wmma.cu:71-104)
 //   kChain  H, Y -> LLR (and Y_eq)       all of them and the demapper; G, C and noiseInv
@@ -38,12 +37,12 @@ namespace aeq {
 // that a warp's reads meet no bank conflicts, and the intermediates' 27.6 MB
 // per 100 MHz slot of HBM traffic are gone from the chain.
 // ---------------------------------------------------------------------------
-enum PlainMode : int { kGram = 0, kCoef = 1, kApply = 2, kChain = 3 };
+enum PlainMode : int { kCoef, kApply, kChain };
 
 struct PlainCell {
     const cf* H;
     const cf* Y;
-    cf* G;              // kGram: out, kCoef: in
+    const cf* G;        // kCoef: in
     cf* C;              // kCoef: out, kApply: in
     float* nInv;        // kCoef: out
     cf* O;              // kApply: out, kChain: optional out
@@ -73,9 +72,9 @@ __host__ __device__ __forceinline__ int plain_cs(int A) { return ((A + 1) & ~1) 
 static int plain_team_bytes(int mode, int A, int L, int S) {
     int v = 0;
     if (mode != kApply) v += A * plain_hs(L);
-    if (mode != kGram) v += L * plain_cs(A);
-    if (mode == kApply || mode == kChain) v += S * plain_cs(A);
-    if (mode == kCoef || mode == kChain) v += L * L + ((3 * L + 1) / 2 + 1);
+    v += L * plain_cs(A);
+    if (mode != kCoef) v += S * plain_cs(A);
+    if (mode != kApply) v += L * L + ((3 * L + 1) / 2 + 1);
     return ((v + 1) & ~1) * (int)sizeof(cf);
 }
 
@@ -95,12 +94,21 @@ __device__ __forceinline__ void cp8(cf* d, const cf* s) {
 }
 __device__ __forceinline__ float4 ld4(const cf* p) { return *reinterpret_cast<const float4*>(p); }
 
-// rows x cols values of src (contiguous) into rows of stride ds.
-template <int TEAM>
+// rows x cols values of src (contiguous) into rows of stride ds.  COLS: cols
+// where known (a divisor of 2 TEAM), so that a lane's pieces lie a constant
+// number of rows apart; else 0.
+template <int TEAM, int COLS = 0>
 __device__ __forceinline__ void stage_rows(cf* dst, int ds, const cf* src, int rows, int cols, int vec, int tid) {
     if (vec) {
         const int half = cols >> 1;
-        if (half >= TEAM) {
+        if constexpr (COLS != 0) {
+            constexpr int HALF = COLS / 2, STEP = TEAM / HALF;
+            static_assert(TEAM % HALF == 0, "a lane keeps its piece of the row");
+            dst += tid / HALF * ds + tid % HALF * 2;
+            src += 2 * tid;
+#pragma unroll 4
+            for (int r = tid / HALF; r < rows; r += STEP, dst += STEP * ds, src += 2 * TEAM) cp16(dst, src);
+        } else if (half >= TEAM) {
             for (int r = 0; r < rows; r++)
                 for (int k = tid; k < half; k += TEAM) cp16(dst + r * ds + 2 * k, src + (long)r * cols + 2 * k);
         } else {
@@ -254,61 +262,25 @@ __global__ void __launch_bounds__(128) plain_kernel(const __grid_constant__ Plai
     const long sc = out ? scw : cl.nSC - 1;
     cf* sH = reinterpret_cast<cf*>(reinterpret_cast<char*>(plain_smem) + (size_t)team * p.teamBytes);
     cf* sC = sH + (MODE != kApply ? A * hs : 0);
-    cf* sY = sC + (MODE != kGram ? L * cs : 0);
-    cf* sL = sY + (MODE == kApply || MODE == kChain ? S * cs : 0);
+    cf* sY = sC + L * cs;
+    cf* sL = sY + (MODE != kCoef ? S * cs : 0);
     float* sInv = reinterpret_cast<float*>(sL + L * L);
     float* sMuInv = sInv + L;
     float* sNoise = sMuInv + L;
 
-    if constexpr (MODE != kApply) stage_rows<TEAM>(sH, hs, cl.H + sc * A * L, A, L, cl.vecH, tid);
+    if constexpr (MODE != kApply) stage_rows<TEAM, EX ? LT : 0>(sH, hs, cl.H + sc * A * L, A, L, cl.vecH, tid);
     else stage_rows<TEAM>(sC, cs, cl.C + sc * A * L, L, A, cl.vecY, tid);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    if constexpr (MODE == kApply || MODE == kChain)
+    if constexpr (MODE != kCoef)
         stage_rows<TEAM>(sY, cs, cl.Y + sc * S * A, S, A, cl.vecY, tid);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     team_sync<TEAM>();
 
-    // ---- G: this lane's row r, columns 2q and 2q + 1 ----
-    // kGram enumerates the whole matrix, the solve its lower triangle (row
-    // pair R holds 2 (R + 1) column pairs, after R (R + 1) of the pairs above).
-    auto gram_pair = [&](int r, int q, cf& g0, cf& g1) {
-        g0 = g1 = make_float2(0.f, 0.f);
-        const cf* hr = sH + r;
-        const cf* hc = sH + 2 * q;
-#pragma unroll 4
-        for (int k = 0; k < A; k++) {
-            const cf v = hr[k * hs];
-            const float4 c = ld4(hc + k * hs);
-            const cf m = make_float2(v.x, -v.y);
-            g0 = cma(m, make_float2(c.x, c.y), g0);
-            g1 = cma(m, make_float2(c.z, c.w), g1);
-        }
-        if (r == 2 * q) g0.x = __fadd_rn(g0.x, cl.sigma2);
-        if (r == 2 * q + 1) g1.x = __fadd_rn(g1.x, cl.sigma2);
-    };
-    if constexpr (MODE == kGram) {
-        constexpr int PR = LT / 2;
-#pragma unroll
-        for (int t = tid; t < LT * PR; t += TEAM) {
-            const int r = t / PR, q = t % PR;
-            if (r >= L || 2 * q >= L) continue;
-            cf g0, g1;
-            gram_pair(r, q, g0, g1);
-            if (!out) continue;
-            cf* g = cl.G + (sc * L + r) * L + 2 * q;
-            if (EX && (reinterpret_cast<uintptr_t>(cl.G) & 15) == 0) {
-                *reinterpret_cast<float4*>(g) = make_float4(g0.x, g0.y, g1.x, g1.y);
-            } else {
-                g[0] = g0;
-                if (2 * q + 1 < L) g[1] = g1;
-            }
-        }
-        return;
-    }
-
     float noise = 0.f;
-    if constexpr (MODE == kCoef || MODE == kChain) {
+    if constexpr (MODE != kApply) {
+        // the lower triangle: row pair R holds 2 (R + 1) column pairs, after
+        // the R (R + 1) of the pairs above
         int R = 0;
         while ((R + 1) * (R + 2) <= tid) R++;
         const int u = tid - R * (R + 1);
@@ -317,7 +289,18 @@ __global__ void __launch_bounds__(128) plain_kernel(const __grid_constant__ Plai
         cf g0 = make_float2(0.f, 0.f), g1 = g0;        // (r, 2q), (r, 2q + 1)
         if (own) {
             if constexpr (MODE == kChain) {
-                gram_pair(r, q, g0, g1);
+                const cf* hr = sH + r;
+                const cf* hc = sH + 2 * q;
+#pragma unroll 4
+                for (int k = 0; k < A; k++) {
+                    const cf v = hr[k * hs];
+                    const float4 c = ld4(hc + k * hs);
+                    const cf m = make_float2(v.x, -v.y);
+                    g0 = cma(m, make_float2(c.x, c.y), g0);
+                    g1 = cma(m, make_float2(c.z, c.w), g1);
+                }
+                if (r == 2 * q) g0.x = __fadd_rn(g0.x, cl.sigma2);
+                if (r == 2 * q + 1) g1.x = __fadd_rn(g1.x, cl.sigma2);
             } else {
                 const cf* g = cl.G + (sc * L + r) * L + 2 * q;
                 g0 = g[0];
@@ -388,7 +371,7 @@ __global__ void __launch_bounds__(128) plain_kernel(const __grid_constant__ Plai
     }
 
     // ---- Y_eq (and LLRs): lane (layer l, symbols st, st + LPL, ...) ----
-    if constexpr (MODE == kApply || MODE == kChain) {
+    if constexpr (MODE != kCoef) {
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         team_sync<TEAM>();
         const int l = tid / LPL, st = tid % LPL;
@@ -399,6 +382,118 @@ __global__ void __launch_bounds__(128) plain_kernel(const __grid_constant__ Plai
             case 2: apply_symbols<MODE, 2, LPL>(cl, sC, sY, cs, noise, sc, l, st, out); break;
             case 3: apply_symbols<MODE, 3, LPL>(cl, sC, sY, cs, noise, sc, l, st, out); break;
             default: apply_symbols<MODE, 4, LPL>(cl, sC, sY, cs, noise, sc, l, st, out); break;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Gram: G[sc][r][c] = sum_k cma(conj(H[k][r]), H[k][c]) (+ sigma2 if r == c):
+// gram_scalar (src/aerial_bottleneck.cu:56-80) with M = H^H, the antenna sum of
+// every element in order.
+//
+// A lane owns RT x CT elements, so its RT + CT operand reads serve RT CT
+// complex products: shared-memory reads return 128 bytes a cycle however many
+// lanes want the same value, and with one row and one column pair a lane
+// (24 bytes for 8 FMAs) they, not the FMA pipe or HBM, set the time.  2 x 2
+// (32 bytes for 16 FMAs; 4 x 4 for 16 layers) puts both near the HBM time of
+// H; 4 x 2 leaves too few warps on an SM (20 KB of H per warp: 22 us).  A warp
+// stages and multiplies its own 32 / lanes subcarriers; a spare row per
+// subcarrier keeps those read together in different banks.  8 slots of 1,584
+// subcarriers x 64 antennas x 8 layers (59 MB): 77 us one thread per element,
+// 22 us one pair per lane, 19 us as here.
+// ---------------------------------------------------------------------------
+constexpr int kGramThreads = 32;
+constexpr int kGramParts = 2;                  // a subcarrier's antennas arrive and are summed in two parts
+__host__ __device__ constexpr int gram_rt(int LT) { return LT == 2 ? 1 : LT == 16 ? 4 : 2; }
+__host__ __device__ constexpr int gram_ct(int LT) { return LT == 16 ? 4 : 2; }
+__host__ __device__ constexpr int gram_team(int LT) { return (LT / gram_rt(LT)) * (LT / gram_ct(LT)); }
+
+struct GramParams {
+    const cf* H;
+    cf* G;
+    float sigma2;
+    int nSC, A, L, vecH, vecG;
+};
+
+template <int LT, bool EX>
+__global__ void __launch_bounds__(kGramThreads) gram_kernel(const GramParams p) {
+    constexpr int RT = gram_rt(LT), CT = gram_ct(LT), TEAM = gram_team(LT), PER = 32 / TEAM;
+    extern __shared__ float4 gram_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int A = p.A, L = EX ? LT : p.L, hs = EX ? LT + 2 : plain_hs(L);
+    const int ts = (A + 1) * hs;                       // values per subcarrier
+    cf* sm = reinterpret_cast<cf*>(gram_smem) + warp * PER * ts;
+    const long sc0 = ((long)blockIdx.x * (blockDim.x >> 5) + warp) * PER;
+    const int n = (int)min((long)PER, (long)p.nSC - sc0);      // subcarriers of this warp
+    const int part = (A + kGramParts - 1) / kGramParts;         // antennas of one copy group
+#pragma unroll
+    for (int q = 0; q < kGramParts; q++) {
+        const int a0 = q * part, rows = min(part, A - a0);
+        for (int j = 0; j < n && rows > 0; j++)
+            stage_rows<32, EX ? LT : 0>(sm + j * ts + a0 * hs, hs, p.H + ((sc0 + j) * A + a0) * L, rows, L, p.vecH, lane);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    const int j = lane / TEAM, t = lane % TEAM;
+    const int r0 = t / (LT / CT) * RT, c0 = t % (LT / CT) * CT;
+    const cf* hr = sm + j * ts + r0;
+    const cf* hc = sm + j * ts + c0;
+    cf acc[RT][CT];
+#pragma unroll
+    for (int i = 0; i < RT; i++)
+#pragma unroll
+        for (int m = 0; m < CT; m++) acc[i][m] = make_float2(0.f, 0.f);
+    auto antennas = [&](int k0, int k1) {
+#pragma unroll 4
+        for (int k = k0; k < k1; k++) {
+            cf rv[RT], cv[CT];
+            if constexpr (RT == 1) {
+                rv[0] = hr[k * hs];
+            } else {
+#pragma unroll
+                for (int i = 0; i < RT; i += 2) {
+                    const float4 v = ld4(hr + k * hs + i);
+                    rv[i] = make_float2(v.x, v.y);
+                    rv[i + 1] = make_float2(v.z, v.w);
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < CT; m += 2) {
+                const float4 v = ld4(hc + k * hs + m);
+                cv[m] = make_float2(v.x, v.y);
+                cv[m + 1] = make_float2(v.z, v.w);
+            }
+#pragma unroll
+            for (int i = 0; i < RT; i++)
+#pragma unroll
+                for (int m = 0; m < CT; m++) acc[i][m] = cma(make_float2(rv[i].x, -rv[i].y), cv[m], acc[i][m]);
+        }
+    };
+    static_assert(kGramParts == 2, "one wait per part");
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncwarp();
+    antennas(0, min(part, A));
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
+    antennas(part, A);
+    if (j >= n || r0 >= L || c0 >= L) return;
+    cf* g = p.G + ((sc0 + j) * L + r0) * L + c0;
+#pragma unroll
+    for (int i = 0; i < RT; i++) {
+        const int r = r0 + i;
+        if (!EX && r >= L) break;
+#pragma unroll
+        for (int m = 0; m < CT; m++)
+            if (r == c0 + m) acc[i][m].x = __fadd_rn(acc[i][m].x, p.sigma2);
+#pragma unroll
+        for (int m = 0; m < CT; m += 2) {
+            if (p.vecG) {                              // L even, G 16-byte aligned
+                if (EX || c0 + m < L)
+                    *reinterpret_cast<float4*>(g + i * L + m) =
+                        make_float4(acc[i][m].x, acc[i][m].y, acc[i][m + 1].x, acc[i][m + 1].y);
+            } else {
+                if (c0 + m < L) g[i * L + m] = acc[i][m];
+                if (c0 + m + 1 < L) g[i * L + m + 1] = acc[i][m + 1];
+            }
         }
     }
 }
@@ -587,20 +682,35 @@ static PlainCell plain_cell(const cf* H, const cf* Y, int nSC, int A, int L, int
     return c;
 }
 
+template <int LT, bool EX>
+static int launch_gram_t(const GramParams& p, cudaStream_t st) {
+    const int s = allow_max_smem<gram_kernel<LT, EX>>();
+    if (s) return s;
+    const size_t warpBytes = (size_t)(32 / gram_team(LT)) * (p.A + 1) * plain_hs(p.L) * sizeof(cf);
+    int warps = kGramThreads / 32;
+    while (warps > 1 && warps * warpBytes > (size_t)kMaxSmemPerCta) warps--;   // one warp needs 131 KB at most
+    const long perBlock = (long)warps * (32 / gram_team(LT));
+    const unsigned blocks = (unsigned)((p.nSC + perBlock - 1) / perBlock);
+    gram_kernel<LT, EX><<<blocks, warps * 32, warps * warpBytes, st>>>(p);
+    return launch_status();
+}
+
 static int launch_gram(const cf* H, float sigma2, cf* G, int nSC, int A, int L, cudaStream_t st) {
-    PlainParams p;
-    p.nCells = 1;
-    p.cell[0] = plain_cell(H, nullptr, nSC, A, L, 1);
-    p.cell[0].G = G;
-    p.cell[0].sigma2 = sigma2;
-    return launch_plain<kGram>(p, st);
+    const bool even = (L % 2) == 0;
+    const GramParams p{H, G, sigma2, nSC, A, L, even && ((uintptr_t)H & 15) == 0, even && ((uintptr_t)G & 15) == 0};
+    switch (layers_tile(L)) {
+        case 2: return L == 2 ? launch_gram_t<2, true>(p, st) : launch_gram_t<2, false>(p, st);
+        case 4: return L == 4 ? launch_gram_t<4, true>(p, st) : launch_gram_t<4, false>(p, st);
+        case 8: return L == 8 ? launch_gram_t<8, true>(p, st) : launch_gram_t<8, false>(p, st);
+        default: return L == 16 ? launch_gram_t<16, true>(p, st) : launch_gram_t<16, false>(p, st);
+    }
 }
 
 static int launch_mmse_coef(const cf* G, const cf* H, cf* C, float* nI, int nSC, int A, int L, cudaStream_t st) {
     PlainParams p;
     p.nCells = 1;
     p.cell[0] = plain_cell(H, nullptr, nSC, A, L, 1);
-    p.cell[0].G = const_cast<cf*>(G);
+    p.cell[0].G = G;
     p.cell[0].C = C;
     p.cell[0].nInv = nI;
     return launch_plain<kCoef>(p, st);
@@ -660,8 +770,18 @@ static int prepare_plain_mode() {
     if (!s) s = prepare_plain_l<MODE, 8>();
     return s ? s : prepare_plain_l<MODE, 16>();
 }
+template <int LT>
+static int prepare_gram() {
+    int s = prepare_one(gram_kernel<LT, true>);
+    if (!s) s = allow_max_smem<gram_kernel<LT, true>>();
+    if (!s) s = prepare_one(gram_kernel<LT, false>);
+    return s ? s : allow_max_smem<gram_kernel<LT, false>>();
+}
 int prepare_plain_kernels() {
-    int s = prepare_plain_mode<kGram>();
+    int s = prepare_gram<2>();
+    if (!s) s = prepare_gram<4>();
+    if (!s) s = prepare_gram<8>();
+    if (!s) s = prepare_gram<16>();
     if (!s) s = prepare_plain_mode<kCoef>();
     if (!s) s = prepare_plain_mode<kApply>();
     if (!s) s = prepare_plain_mode<kChain>();
