@@ -35,15 +35,14 @@ namespace aeq {
 
 constexpr int kMaxCells = AERIAL_MAX_CELLS;
 
-// Subcarriers per group: GS = min(32 / LT, cap).  32 / LT fills every lane
-// of the FP32 solve and of the LLR epilogue (LT lanes per subcarrier); a
-// smaller cap shortens each group's operand pass (GS x chunks items), which
-// an uneven batch needs so that no warp is left with a few long groups: on
-// the uneven 16-cell batch a cap of 4 (idle solve lanes on 1-, 2- and
-// 4-layer tiles) measured 54.3 us against 66.6 us for a cap of 8.
-// The cap is a tuning parameter (aerial_tuning.sc_per_group, searched by the
-// autotuner).
-constexpr int kDefaultGroupCap = 4;
+// Subcarriers per group (set_groups): at most 32 / LT, which fills every lane
+// of the FP32 solve and of the LLR epilogue (LT lanes per subcarrier), and at
+// most a cap: aerial_tuning.sc_per_group, searched by the autotuner, or these
+// where it is 0.  The uniform batches' kernels hand out groups dynamically
+// and run best with the solve's lanes full at 8 layers and short groups below
+// (16 cells of 273 PRB, 4 layers, 64 antennas: 85 us at 4, 93 us at 8).
+constexpr int kUniformGroupCap = 4;
+constexpr int kMixedGroupCap = 8;
 
 struct FusedCell {
     const float2* H;
@@ -54,7 +53,7 @@ struct FusedCell {
     float sigma2;    // noise variance in the units the kernel sees (times scale^2)
     float scale;     // power-of-two operand scale (FP16 operands), else 1
     int nSC, A, L, nSym, nPam, LT, vecY, vecH, lgHalfL;
-    int GS;          // subcarriers per group = min(32 / LT, group cap)
+    int GS;          // subcarriers per group (set_groups)
     int nChunk;      // 16-antenna chunks per subcarrier
     int hrs;         // staged channel-row stride (bytes)
     PamLut lut;
@@ -1750,24 +1749,62 @@ extern "C" float aerial_fp16_operand_scale(float sigma2) {
 
 namespace aeq {
 
-// Group size of every cell (min(32 / LT, cap)) and the first group index of
-// each, in launch order.  Warps take groups round-robin (warp w: groups w,
-// w + nw, ...).  Measured on the uneven 16-cell batch (configuration 4), same
-// box, against this walk with cap 4 (54.3 us): a snake walk over cells sorted
-// by estimated group cost 56.3 us, sorting alone 56.3-58.3 us, cap 8 with the
-// plain walk 66.6 us; the autotuner's launch shapes recover 54.3 us in every
-// variant, and no variant beats the plain walk.  Outputs are bit-identical
-// across all of them.
-void set_groups(FusedParams& p, int cap) {
-    if (cap < 1) cap = kDefaultGroupCap;
+// Group sizes and the first group index of each cell, in launch order.  `warps`
+// is the number the launch keeps resident; warp w takes groups w, w + warps, ...
+// (mixed kernels) or w and then the next free one (uniform ones).
+//
+// A launch ends with the warp that holds the most work, and a group's time is
+// its chain of (subcarrier, 16-antenna chunk) items, each a wait for memory,
+// plus one solve.  So a launch with few subcarriers gives every group its own
+// warp and makes the groups as short as that allows, and in a batch of
+// different cells groups are made equal in items, not in subcarriers (with
+// four subcarriers a group, one of a 64-antenna cell is four times as long as
+// one of a 16-antenna cell in the same round).  Where even groups of
+// kMaxItems items do not fit the resident warps at once, kRoundItems a group
+// balances the rounds against the solves, whose cost is per group.
+//
+// Measured back to back, subcarriers per group 4 everywhere -> this rule:
+// one slot of 24 PRB x 32 antennas x 4 layers 8.3 -> 6.3 us, two of
+// 132 x 64 x 8 16.5 -> 14.5, one of 100 PRB x 48 x 3 16.5 -> 10.4; mixed
+// batches of 8 / 16 / 48 cells 32.9 -> 27 / 34 -> 33 / 112 -> 103 us, of 24
+// and 48 cells with ragged shapes 72 -> 53 and 114 -> 106 us.  Over 58 random
+// batches of 1 to 64 cells it is 2 % off the best of 13 item counts (geometric
+// mean), four subcarriers a group 22 %; 8 or 16 items in the rounds' place
+// 3.6 % and 2.8 %.  One subcarrier a group in a uniform batch keeps most
+// lanes of the solve idle and pays only while half the warps are free (one
+// slot of 132 x 64 x 8: 10.9 us at 1, 10.3 us at 2).
+// A subcarrier's results do not depend on its group.
+constexpr int kMaxItems = 16, kRoundItems = 12;
+
+static long assign_groups(FusedParams& p, int items, int fixed, int cap) {
     long g0 = 0;
     for (int i = 0; i < p.nCells; i++) {
         FusedCell& f = p.cell[i];
-        f.GS = 32 / f.LT < cap ? 32 / f.LT : cap;
+        const int most = 32 / f.LT < cap ? 32 / f.LT : cap;
+        const int gs = fixed ? fixed : (items + f.nChunk / 2) / f.nChunk;
+        f.GS = gs < 1 ? 1 : gs > most ? most : gs;
         f.group0 = g0;
         g0 += (f.nSC + f.GS - 1) / f.GS;
     }
     p.totalGroups = g0;
+    return g0;
+}
+
+void set_groups(FusedParams& p, int cap, long warps) {
+    if (p.exactChunks) {                              // uniform batch
+        if (cap < 1) cap = kUniformGroupCap;
+        for (int gs = 1; gs < cap; gs *= 2)
+            if (assign_groups(p, 0, gs, cap) <= (gs == 1 ? warps / 2 : warps)) return;
+        assign_groups(p, 0, cap, cap);
+        return;
+    }
+    if (cap < 1) cap = kMixedGroupCap;
+    long subcarriers = 0;
+    for (int i = 0; i < p.nCells; i++) subcarriers += p.cell[i].nSC;
+    if (subcarriers <= warps * cap)                   // else no grouping fits one round
+        for (int items : {1, 2, 3, 4, 5, 6, 8, 10, 12, kMaxItems})
+            if (assign_groups(p, items, 0, cap) <= warps) return;
+    assign_groups(p, kRoundItems, 0, cap);
 }
 
 // warpBytes: the per-warp shared memory of the launch (epilogue region of the
@@ -1814,7 +1851,7 @@ int build_fused_params(const aerial_cell_desc* cells, int nCells, FusedParams& p
     p.nCells = nCells;
     p.scaled = 0;
     p.walkSlot = -1;
-    set_groups(p, kDefaultGroupCap);
+    p.totalGroups = 0;              // set_groups decides, once the launch shape is known
     p.fmt = cells[0].format;
     for (int i = 0; i < nCells; i++)
         if (cells[i].format != p.fmt || (p.fmt != AERIAL_FMT_CF32 && p.fmt != AERIAL_FMT_CF16))
@@ -1909,6 +1946,7 @@ void set_operand_scale(FusedParams& p, int prec) {
 struct LaunchShape {
     int warps, ctasPerSm;
 };
+static long resident_warps(LaunchShape sh) { return (long)sm_count() * sh.ctasPerSm * sh.warps; }
 
 // Launch shapes are limited by 16 resident warps per SM (128 registers per
 // thread) and by shared memory (operand ring + epilogue region per warp).
@@ -2115,7 +2153,10 @@ static WalkTable* walk_table_locked(std::unique_lock<std::mutex>& lk, int* devOu
 // uneven 16-cell batch that measured slower (57.4-58.2 against 54.3 us; with
 // the ticket taken a whole group ahead still 58.4 against 54.2 us), so they
 // keep the static walk.
-static bool walk_applies(const FusedParams& p) { return p.exactChunks != 0 && !p.halfMixed; }
+// A launch whose warps hold one group each at most never asks for a ticket.
+static bool walk_applies(const FusedParams& p, const LaunchPlan& pl) {
+    return p.exactChunks != 0 && !p.halfMixed && p.totalGroups > (long)pl.grid.x * (pl.block.x / 32);
+}
 
 static bool walk_slot_idle(WalkSlot& w) {
     if (!w.last) return true;
@@ -2166,7 +2207,7 @@ int launch_fused(FusedParams& p, int warpBytes, int prec, LaunchShape sh, cudaSt
     int s = plan_fused(p, warpBytes, prec, sh, pl);
     if (s) return s;
     std::unique_lock<std::mutex> lk;
-    WalkTable* t = walk_applies(p) ? walk_table_locked(lk) : nullptr;
+    WalkTable* t = walk_applies(p, pl) ? walk_table_locked(lk) : nullptr;
     p.walkSlot = t ? walk_slot_for_stream(t, st) : -1;
     void* args[] = {&p};
     const cudaError_t e = cudaLaunchKernel(pl.func, pl.grid, pl.block, args, (size_t)pl.smem, st);
@@ -2181,7 +2222,7 @@ int launch_fused(FusedParams& p, int warpBytes, int prec, LaunchShape sh, cudaSt
 static void resolve_tuning(const aerial_tuning* tuning, int warpBytes, int& prec, LaunchShape& sh, int& gsCap) {
     sh = default_shape(warpBytes);
     prec = AERIAL_PREC_FP16;
-    gsCap = kDefaultGroupCap;
+    gsCap = 0;
     if (tuning) {
         prec = tuning->precision;
         if (tuning->sc_per_group > 0) gsCap = tuning->sc_per_group;
@@ -2207,14 +2248,14 @@ extern "C" int aerial_pusch_eq_fused(const aerial_cell_desc* cells, int nCells, 
     LaunchShape sh;
     int prec, gsCap;
     resolve_tuning(tuning, warpBytes, prec, sh, gsCap);
-    if (gsCap != kDefaultGroupCap) set_groups(p, gsCap);
+    set_groups(p, gsCap, resident_warps(sh));
     set_operand_scale(p, prec);
     return launch_fused(p, warpBytes, prec, sh, to_stream(stream));
 }
 
 // ---------------------------------------------------------------------------
 // Autotuner: time each candidate tile and launch shape on the caller's cells
-// and keep the fastest.  Candidates are the group cap (subcarriers solved
+// and keep the fastest.  Candidates are the group cap (most subcarriers solved
 // together per warp: 4, 8 or 32, for batches with tiles of 4 layers or fewer,
 // where the cap changes anything) crossed with (warps per CTA, CTAs per SM)
 // pairs whose shared memory fits one SM; each is timed with CUDA events over
@@ -2234,7 +2275,7 @@ extern "C" int aerial_autotune(const aerial_cell_desc* cells, int nCells, aerial
         LaunchShape sh;
         int cap;
     };
-    int caps[3] = {kDefaultGroupCap, 0, 0}, nCaps = 1;
+    int caps[3] = {kUniformGroupCap, 0, 0}, nCaps = 1;
     bool smallTile = false;
     for (int i = 0; i < base.nCells; i++) smallTile |= base.cell[i].LT <= 4;
     if (smallTile) {
@@ -2267,8 +2308,8 @@ extern "C" int aerial_autotune(const aerial_cell_desc* cells, int nCells, aerial
     for (int rd = 0; rd < rounds && !s; rd++) {
         for (int ic = 0; ic < nc && !s; ic++) {
             const LaunchShape& sh = cand[ic].sh;
-            p = base;                                // unscaled sigma2, default groups
-            set_groups(p, cand[ic].cap);
+            p = base;                                // unscaled sigma2
+            set_groups(p, cand[ic].cap, resident_warps(sh));
             set_operand_scale(p, prec);
             if ((s = launch_fused(p, warpBytes, prec, sh, st))) break;
             cudaEventRecord(e0, st);
@@ -2288,14 +2329,14 @@ extern "C" int aerial_autotune(const aerial_cell_desc* cells, int nCells, aerial
     }
     float fastest = 1e30f;
     for (int ic = 0; ic < nc; ic++) fastest = t[ic] < fastest ? t[ic] : fastest;
-    Cand bestC{def, kDefaultGroupCap};
+    Cand bestC{def, kUniformGroupCap};
     float bestT = 1e30f;
     int bestWarps = -1;
     for (int ic = 0; ic < nc; ic++) {
         if (t[ic] > fastest * 1.02f) continue;
         const int w = cand[ic].sh.warps * cand[ic].sh.ctasPerSm;
         const bool better = w > bestWarps ||
-                            (w == bestWarps && cand[ic].cap == kDefaultGroupCap && bestC.cap != kDefaultGroupCap) ||
+                            (w == bestWarps && cand[ic].cap == kUniformGroupCap && bestC.cap != kUniformGroupCap) ||
                             (w == bestWarps && cand[ic].cap == bestC.cap && t[ic] < bestT);
         if (better) {
             bestWarps = w;
@@ -2328,7 +2369,7 @@ struct aerial_eq_graph {
     LaunchPlan plan;
     int prec = AERIAL_PREC_FP16;
     LaunchShape shape{};
-    int gsCap = kDefaultGroupCap;
+    int gsCap = 0;
     int dev = -1;                    // device of the graph's walk slot (params.walkSlot)
     WalkTable* walk = nullptr;       // table of that slot
 };
@@ -2360,14 +2401,14 @@ extern "C" int aerial_eq_graph_create(const aerial_cell_desc* cells, int nCells,
     int s = build_fused_params(cells, nCells, g->params, warpBytes);
     if (!s) {
         resolve_tuning(tuning, warpBytes, g->prec, g->shape, g->gsCap);
-        if (g->gsCap != kDefaultGroupCap) set_groups(g->params, g->gsCap);
+        set_groups(g->params, g->gsCap, resident_warps(g->shape));
         set_operand_scale(g->params, g->prec);
         s = plan_fused(g->params, warpBytes, g->prec, g->shape, g->plan);
     }
     if (!s) {
         // the graph's own walk slot: its replays are ordered among themselves
         std::unique_lock<std::mutex> lk;
-        WalkTable* t = walk_applies(g->params) ? walk_table_locked(lk, &g->dev) : nullptr;
+        WalkTable* t = walk_applies(g->params, g->plan) ? walk_table_locked(lk, &g->dev) : nullptr;
         int held = 0;                // graphs hold at most kWalkSlots - 16: streams keep slots
         for (int k = 0; t && k < kWalkSlots; k++) held += t->s[k].graph ? 1 : 0;
         const int i = t && held < kWalkSlots - 16 ? walk_free_slot(t) : -1;
@@ -2413,7 +2454,7 @@ extern "C" int aerial_eq_graph_update(aerial_eq_graph* g, const aerial_cell_desc
     // The new noise levels may move a cell in or out of FP16 operand scaling,
     // which selects another kernel instantiation: re-plan the node (an
     // executable graph's kernel node may change its function).
-    if (g->gsCap != kDefaultGroupCap) set_groups(np, g->gsCap);
+    set_groups(np, g->gsCap, resident_warps(g->shape));
     set_operand_scale(np, g->prec);
     np.walkSlot = g->params.walkSlot;
     LaunchPlan pl;

@@ -263,9 +263,11 @@ typedef struct {
     int warps_per_cta;         /* 0 = default */
     int ctas_per_sm;           /* 0 = default */
     int sc_per_group;          /* cap on the subcarriers a warp solves together
-                                  (min(32 / layer tile, cap)); 0 = default (4:
-                                  short groups, so no warp of an uneven batch
-                                  is left with a few long ones) */
+                                  (at most min(32 / layer tile, cap); fewer
+                                  where the launch is small or a cell has many
+                                  antennas, so that no warp is left with a few
+                                  long groups); 0 = default (4 for uniform
+                                  batches, 8 for mixed ones) */
 } aerial_tuning;
 
 /* Equalize nCells cell-slots in ONE persistent launch (cells may differ in
