@@ -53,6 +53,8 @@ struct FusedCell {
     float sigma2;    // noise variance in the units the kernel sees (times scale^2)
     float scale;     // power-of-two operand scale (FP16 operands), else 1
     int nSC, A, L, nSym, nPam, LT, vecY, vecH, lgHalfL;
+    int vecRun;      // every subcarrier's channel starts on 16 bytes
+    int exact;       // mixed kernel: L fills its tile, whole chunks, aligned rows
     int GS;          // subcarriers per group (set_groups)
     int nChunk;      // 16-antenna chunks per subcarrier
     int hrs;         // staged channel-row stride (bytes)
@@ -281,6 +283,10 @@ constexpr int CHUNK = 16;       // antennas per stage (two k-steps)
 __host__ __device__ constexpr int hrs_of(int L) {
     return (((8 * L + 15) & ~15) + 16) < 48 ? 48 : (((8 * L + 15) & ~15) + 16);
 }
+// Channel-row stride of a mixed launch: padded for L = 2, 4, 8, 16, whose rows
+// would fall in the same banks, and the row itself for the others (which
+// spread over the banks by themselves, at most two to a bank).
+__host__ __device__ constexpr int hrs_any(int L) { return L > 1 && (L & (L - 1)) == 0 ? hrs_of(L) : 8 * L; }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(__cvta_generic_to_global(src))
@@ -288,6 +294,17 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(__cvta_generic_to_global(src))
+                 : "memory");
+}
+// The same with only the first `bytes` read and the rest of the piece zeroed.
+__device__ __forceinline__ void cp_async16z(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(__cvta_generic_to_global(src)),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async8z(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(__cvta_generic_to_global(src)),
+                 "r"(bytes)
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
@@ -309,9 +326,11 @@ __device__ __forceinline__ float4 lds128(uint32_t a) {
 // Fragment reads of one staged chunk (two k-steps) and their MMAs.  Thread
 // (g, c) of k-step kk owns the antenna pair 8kk + 2c, +1 of the chunk.
 //
-// FULL: all 16 antennas of the chunk exist, so no antenna mask is applied.
-// Rows of symbols past nSym are never masked: each received row only feeds
-// its own Z column, and columns past nSym are never read.
+// Nothing is masked here.  Antennas past the array are zero rows in the stage
+// (the copies fill them in; FULL = false only skips a k-step without any),
+// layers past L read whatever follows their row and feed rows and columns of
+// G and Z that solve_group replaces or never reads, and rows of symbols past
+// nSym feed Z columns that are never read.
 // yo[kk][nt]: the lane's received-row fragment offsets in a stage (row
 // 8 nt + g, clamped to row 0 past nSym, antenna pair 8 kk + 2 c, swizzled),
 // fixed per cell.
@@ -319,33 +338,26 @@ __device__ __forceinline__ float4 lds128(uint32_t a) {
 // raw FP16 is safe are multiplied by the cell's power-of-two scale ss = (s, s)
 // before they are rounded (exact; the cell's sigma2 carries s^2, so G^-1 Z,
 // mu and the LLRs are unchanged).
-template <int LT, int P, bool LEXACT, bool FULL, bool SC = false>
-__device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, int L, const uint32_t (&yo)[2][2],
+template <int LT, int P, bool FULL, bool SC = false>
+__device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, const uint32_t (&yo)[2][2],
                                           float (*gacc)[4], float (*zacc)[2][4], bool z2, int g, int c,
                                           unsigned long long ss = 0) {
     constexpr int NMT = LT > 8 ? 2 : 1;
 #pragma unroll
     for (int kk = 0; kk < 2; kk++) {
         const int a0 = 8 * kk + 2 * c;
-        if (!FULL && 8 * kk >= nRows) break;             // uniform: tail chunk of 8 antennas
-        const bool v0 = FULL || a0 < nRows, v1 = FULL || a0 + 1 < nRows;
+        if (!FULL && 8 * kk >= nRows) break;             // uniform: tail chunk of 8 antennas or fewer
         float4 hv[NMT];
 #pragma unroll
         for (int mt = 0; mt < NMT; mt++) {
             const int l = g + 8 * mt;
-            const bool lv = LEXACT || l < L;             // LEXACT: every lane's layer exists (L == LT)
-            const int la = lv ? l : 0;                   // padded layers read row data they then discard
-            const float2 h0 = lds64(st + a0 * hrs + la * 8);
-            const float2 h1 = lds64(st + (a0 + 1) * hrs + la * 8);
-            hv[mt] = make_float4((lv && v0) ? h0.x : 0.f, (lv && v0) ? h0.y : 0.f, (lv && v1) ? h1.x : 0.f,
-                                 (lv && v1) ? h1.y : 0.f);
+            const float2 h0 = lds64(st + a0 * hrs + l * 8);
+            const float2 h1 = lds64(st + (a0 + 1) * hrs + l * 8);
+            hv[mt] = make_float4(h0.x, h0.y, h1.x, h1.y);
         }
         float4 yv[2];
 #pragma unroll
-        for (int nt = 0; nt < 2; nt++) {
-            const float4 y = lds128(st + yo[kk][nt]);
-            yv[nt] = FULL ? y : make_float4(v0 ? y.x : 0.f, v0 ? y.y : 0.f, v1 ? y.z : 0.f, v1 ? y.w : 0.f);
-        }
+        for (int nt = 0; nt < 2; nt++) yv[nt] = lds128(st + yo[kk][nt]);
         if constexpr (SC) {
 #pragma unroll
             for (int mt = 0; mt < NMT; mt++) hv[mt] = scale4(hv[mt], ss);
@@ -415,8 +427,11 @@ __device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, int L
 // Accumulators of subcarrier q of the group -> per-warp shared memory.
 // Fragment (row g, cols 2c, 2c+1) and (row g+8, ...) = Re / Im of
 // out[8mt+g][8nt+2c], out[8mt+g][8nt+2c+1]: one 16-byte store each.
+// L: layers; Z rows past L are stored as zeros, because X = G^-1 Z multiplies
+// them (by zeros of G^-1) and what was summed there may not be finite.
 template <int LT>
-__device__ __forceinline__ void store_acc(float2* sm, float (*gacc)[4], float (*zacc)[2][4], int q, int g, int c) {
+__device__ __forceinline__ void store_acc(float2* sm, float (*gacc)[4], float (*zacc)[2][4], int q, int g, int c,
+                                          int L = LT) {
     using W = WarpSmem<LT>;
     constexpr int NMT = LT > 8 ? 2 : 1;
     float2* sG = sm + W::offG + q * W::GB;
@@ -435,7 +450,9 @@ __device__ __forceinline__ void store_acc(float2* sm, float (*gacc)[4], float (*
         for (int nt = 0; nt < 2; nt++) {
             const float* d = zacc[mt][nt];
             const int s = 8 * nt + 2 * c;
-            if (r < LT) *reinterpret_cast<float4*>(sZ + r * W::ZS + s) = make_float4(d[0], d[2], d[1], d[3]);
+            if (r < LT)
+                *reinterpret_cast<float4*>(sZ + r * W::ZS + s) =
+                    r < L ? make_float4(d[0], d[2], d[1], d[3]) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
 }
@@ -626,7 +643,9 @@ __device__ __forceinline__ void get_row(const float2* row, float2 (&b)[LT]) {
 // warp's epilogue region: LT lanes per subcarrier.
 // ---------------------------------------------------------------------------
 // H16: Y_eq and LLRs are stored as half precision (the FP16 I/O format).
-template <int LT, int P, bool H16 = false>
+// PAD: cells may have fewer than LT layers; columns past L of the rows that
+// exist are then cleared.
+template <int LT, int P, bool H16 = false, bool PAD = false>
 __device__ __noinline__ void solve_group(const CellView cl, long sc0, int nValid, int smemOff, int lane) {
     using W = WarpSmem<LT>;
     extern __shared__ float4 smem_raw[];
@@ -662,7 +681,7 @@ __device__ __noinline__ void solve_group(const CellView cl, long sc0, int nValid
     }
 #pragma unroll
     for (int m = 0; m < LT; m++) {
-        float2 v = (scValid && real) ? r[m] : make_float2(0.f, 0.f);
+        float2 v = (scValid && real && (!PAD || m < cl.L)) ? r[m] : make_float2(0.f, 0.f);
         if (m == i) v = real ? make_float2(v.x + s2, 0.f) : make_float2(1.f, 0.f);
         r[m] = v;
     }
@@ -764,7 +783,8 @@ __device__ __noinline__ void solve_group(const CellView cl, long sc0, int nValid
 inline int stage_bytes_of(const FusedParams& p) {
     int b = 0;
     for (int ci = 0; ci < p.nCells; ci++) {
-        const int v = CHUNK * hrs_of(p.cell[ci].L) + 128 * p.cell[ci].nSym;
+        // layers past L of the last rows read up to 128 bytes past the channel rows
+        const int v = CHUNK * p.cell[ci].hrs + 128 * p.cell[ci].nSym;
         b = v > b ? v : b;
     }
     return (b + 15) & ~15;
@@ -778,88 +798,72 @@ inline int epi_bytes_of(const FusedParams& p) {
     return (b + 15) & ~15;
 }
 
-// Stage the copies of one item (subcarrier base pointers hs / ys, chunk ch)
-// of cell cl into the stage at shared address st.  Subcarriers of a group
-// are contiguous, so the producer only advances pointers between items.
-__device__ __forceinline__ void stage_item(const FusedCell& cl, const float2* hs, const float2* ys, int ch,
-                                           uint32_t st, int lane) {
-    const int L = cl.L, A = cl.A, nSym = cl.nSym, hrs = cl.hrs;
-    const int nRows = min(CHUNK, A - CHUNK * ch);
-    const float2* hsrc = hs + CHUNK * ch * L;
-    if (cl.vecH) {                      // L even: 16-byte pieces, L/2 per row
-        const int half = L >> 1;
-        const int n = nRows * half;
-        if (cl.lgHalfL >= 0) {
-            const int sh = cl.lgHalfL;
-            for (int e = lane; e < n; e += 32) cp_async16(st + (e >> sh) * hrs + (e & (half - 1)) * 16, hsrc + 2 * e);
+// Bytes of a 16-byte piece at byte `at` of `valid` bytes.
+__device__ __forceinline__ int piece_bytes(int valid, int at) { return min(16, max(0, valid - at)); }
+
+// The received rows of one chunk of nRows antennas at ys (the subcarrier's
+// row 0, the chunk's first antenna): rows lane / 8 + 4 k, piece lane % 8,
+// zeros past the last antenna.
+__device__ __forceinline__ void stage_rows_y(uint32_t yst, const float2* ys, int A, int nSym, int nRows, int vecY,
+                                             int lane) {
+    const int s0 = lane >> 3, a = 2 * (lane & 7);
+    const uint32_t d0 = yst + s0 * 128 + (((lane & 7) ^ ((s0 & 1) << 2)) << 4);
+    const int bytes = piece_bytes(8 * nRows, 8 * a);
+    const float2* src = ys + (long)s0 * A + (bytes ? a : 0);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (s0 + 4 * k >= nSym) break;
+        const uint32_t d = d0 + 512 * k;
+        if (vecY) {
+            cp_async16z(d, src, bytes);
         } else {
-            for (int e = lane; e < n; e += 32) {
-                const int row = e / half;
-                cp_async16(st + row * hrs + (e - row * half) * 16, hsrc + 2 * e);
-            }
+            cp_async8z(d, src, min(8, bytes));
+            cp_async8z(d + 8, src + (bytes > 8 ? 1 : 0), max(0, bytes - 8));
         }
-    } else {                            // 8-byte pieces
-        const int n = nRows * L;
-        for (int e = lane; e < n; e += 32) {
-            const int row = e / L;
-            cp_async8(st + row * hrs + (e - row * L) * 8, hsrc + e);
-        }
-    }
-    const uint32_t yst = st + CHUNK * hrs;
-    const float2* ysrc = ys + CHUNK * ch;
-    for (int e = lane; e < nSym * 8; e += 32) {
-        const int s = e >> 3, k = e & 7;
-        const int a = 2 * k;
-        if (a < nRows) {
-            const uint32_t d = yst + s * 128 + ((k ^ ((s & 1) << 2)) << 4);
-            const float2* src = ysrc + (long)s * A + a;
-            if (cl.vecY && a + 1 < nRows) {
-                cp_async16(d, src);
-            } else {
-                cp_async8(d, src);
-                if (a + 1 < nRows) cp_async8(d + 8, src + 1);
-            }
-        }
+        src += 4 * A;
     }
 }
 
-// stage_item for a launch whose cells all have L == LF (even): strides and
-// piece mapping are compile-time constants.
+// One chunk of nRows antennas of any cell: hs / ys point at its first channel
+// value and its first received value.  A subcarrier's channel is one run of
+// bytes, so its pieces go out in order without a division by L (whose rows are
+// not padded unless L is a power of two, see hrs_any); a run that is only
+// 8-byte aligned goes in 8-byte pieces.
+__device__ __forceinline__ void stage_any(const FusedCell& cl, const float2* hs, const float2* ys, int nRows,
+                                          uint32_t st, int lane) {
+    const int L = cl.L, pad = cl.hrs - 8 * L;
+    const int valid = 8 * L * nRows;                   // bytes of channel that exist
+    const int rows = nRows > 8 ? CHUNK : 8;            // rows the MMAs read
+    if (cl.vecRun) {
+        for (int e = lane; 2 * e < rows * L; e += 32) {
+            const int bytes = piece_bytes(valid, 16 * e);
+            cp_async16z(st + 16 * e + (pad ? (e >> cl.lgHalfL) * pad : 0), hs + (bytes ? 2 * e : 0), bytes);
+        }
+    } else {
+        for (int e = lane; e < rows * L; e += 32) {
+            const int bytes = 8 * e < valid ? 8 : 0;
+            cp_async8z(st + 8 * e + (pad ? ((2 * e) >> (cl.lgHalfL + 2)) * pad : 0), hs + (bytes ? e : 0), bytes);
+        }
+    }
+    stage_rows_y(st + CHUNK * cl.hrs, ys, cl.A, cl.nSym, nRows, cl.vecY, lane);
+}
+
+// stage_any for a launch whose cells all have L == LF (even) and aligned rows:
+// strides and piece mapping are compile-time constants.
 template <int LF>
 __device__ __forceinline__ void stage_item_exact(const FusedCell& cl, const float2* hs, const float2* ys, int ch,
                                                  uint32_t st, int lane) {
     constexpr int HRS = hrs_of(LF);
     constexpr int HALF = LF / 2;
-    const int A = cl.A, nSym = cl.nSym;
-    const int nRows = min(CHUNK, A - CHUNK * ch);
+    const int nRows = min(CHUNK, cl.A - CHUNK * ch);
     const float2* hsrc = hs + CHUNK * ch * LF;
-    const int n = nRows * HALF;
 #pragma unroll
     for (int k = 0; k < (CHUNK * HALF + 31) / 32; k++) {
         const int e = lane + 32 * k;
-        if (e < n) cp_async16(st + (e / HALF) * HRS + (e % HALF) * 16, hsrc + 2 * e);
+        const bool in = e < nRows * HALF;
+        if (e < CHUNK * HALF) cp_async16z(st + (e / HALF) * HRS + (e % HALF) * 16, hsrc + (in ? 2 * e : 0), in ? 16 : 0);
     }
-    const uint32_t yst = st + CHUNK * HRS;
-    const float2* ysrc = ys + CHUNK * ch;
-    if (nRows == CHUNK) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) {                  // up to 16 rows x 8 pieces
-            const int e = lane + 32 * k;
-            const int s = e >> 3, kk = e & 7;
-            if (s < nSym) cp_async16(yst + s * 128 + ((kk ^ ((s & 1) << 2)) << 4), ysrc + (long)s * A + 2 * kk);
-        }
-    } else {
-        for (int e = lane; e < nSym * 8; e += 32) {
-            const int s = e >> 3, kk = e & 7;
-            const int a = 2 * kk;
-            if (a < nRows) {
-                const uint32_t d = yst + s * 128 + ((kk ^ ((s & 1) << 2)) << 4);
-                const float2* src = ysrc + (long)s * A + a;
-                if (a + 1 < nRows) cp_async16(d, src);
-                else cp_async8(d, src);
-            }
-        }
-    }
+    stage_rows_y(st + CHUNK * HRS, ys + CHUNK * ch, cl.A, cl.nSym, nRows, 1, lane);
 }
 
 // A full 16-antenna chunk of a launch whose cells all have L == LF: the
@@ -887,9 +891,9 @@ __device__ __forceinline__ int group_valid(const FusedCell& cl, long grp) {
     return (int)min((long)cl.GS, (long)cl.nSC - (grp - cl.group0) * cl.GS);
 }
 
-// LTF = 0: any mix of cells.  LTF in {2, 4, 8, 16}: every cell has
-// nLayers == LTF and 16-byte aligned H / Y_rx (the host checks), so the layer
-// tile, strides and masks are compile-time constants.
+// LTF in {2, 4, 8, 16}: every cell has nLayers == LTF and 16-byte aligned H /
+// Y_rx (the host checks), so the layer tile and strides are compile-time
+// constants.
 // SC: the launch has cells whose FP16 operands are scaled (mma_stage).
 template <int P, int LTF, bool SC = false>
 __global__ void __launch_bounds__(256, 2) fused_eq_kernel(const __grid_constant__ FusedParams p) {
@@ -910,20 +914,16 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel(const __grid_constant_
     if (gw >= total) return;
 
     // ---- producer cursor (registers): group, cell, subcarrier, chunk ----
-    // Per-lane staging offsets are fixed for the whole launch (exact tile) or
-    // for a cell (received-row pieces), so a full chunk costs a few adds and
+    // Per-lane staging offsets are fixed for the whole launch (channel pieces)
+    // or for a cell (received-row pieces), so a full chunk costs a few adds and
     // its cp.async instructions.
-    uint32_t hLaneS = 0, yLaneS = 0;
-    if constexpr (LTF != 0) {
-        constexpr int HALF = LTF / 2;
-        hLaneS = (lane / HALF) * hrs_of(LTF) + (lane % HALF) * 16;
-        yLaneS = CHUNK * hrs_of(LTF) + (lane >> 3) * 128 + (((lane & 7) ^ (((lane >> 3) & 1) << 2)) << 4);
-    }
+    constexpr int HALF = LTF / 2;
+    const uint32_t hLaneS = (lane / HALF) * hrs_of(LTF) + (lane % HALF) * 16;
+    const uint32_t yLaneS = CHUNK * hrs_of(LTF) + (lane >> 3) * 128 + (((lane & 7) ^ (((lane >> 3) & 1) << 2)) << 4);
     long pg = gw;
     int pci = 0;
     while (pci + 1 < p.nCells && pg >= p.cell[pci + 1].group0) pci++;
     int pq = 0, pch = 0, pslot = 0, pValid, pNChunk, pNFull, pYStep, pYLane, pYk;
-    int pExact = 0;                                       // generic kernel: this cell's exact tile, or 0
     long pHsc, pYsc;
     const float2* phs;
     const float2* pys;
@@ -932,7 +932,7 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel(const __grid_constant_
         const int A = cl.A, nSym = cl.nSym;
         pNChunk = cl.nChunk;
         pNFull = A / CHUNK;
-        pHsc = (long)A * (LTF != 0 ? LTF : cl.L);
+        pHsc = (long)A * LTF;
         pYsc = (long)nSym * A;
         pValid = group_valid(cl, pg);
         const long sc = (pg - cl.group0) * cl.GS;
@@ -941,41 +941,16 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel(const __grid_constant_
         pYStep = 4 * A;                                   // received rows s and s + 4
         pYLane = (lane >> 3) * A + 2 * (lane & 7);        // this lane's first piece
         pYk = min(4, max(0, (nSym - (lane >> 3) + 3) >> 2));
-        if constexpr (LTF == 0) {
-            // a cell whose layers fill its tile stages full chunks like the
-            // exact-tile kernels, with this cell's lane offsets
-            pExact = (cl.L == cl.LT && cl.LT >= 2 && cl.vecH && cl.vecY) ? cl.LT : 0;
-            if (pExact) {
-                const int half = cl.L / 2;
-                hLaneS = (lane / half) * cl.hrs + (lane % half) * 16;
-                yLaneS = CHUNK * cl.hrs + (lane >> 3) * 128 + (((lane & 7) ^ (((lane >> 3) & 1) << 2)) << 4);
-            }
-        }
     };
     load_pcell();
     auto produce = [&]() {
         if (pg < total) {
             const uint32_t st = stBase + pslot * p.stageBytes;
-            if constexpr (LTF != 0) {
-                if (pch < pNFull)
-                    stage_full<LTF>(st, hLaneS, yLaneS, phs + CHUNK * pch * LTF, pys + CHUNK * pch + pYLane, pYStep,
-                                    pYk, lane);
-                else
-                    stage_item_exact<LTF>(p.cell[pci], phs, pys, pch, st, lane);
-            } else {
-                if (pExact && pch < pNFull) {
-                    const float2* hsrc = phs + CHUNK * pch * pExact;
-                    const float2* ysrc = pys + CHUNK * pch + pYLane;
-                    switch (pExact) {
-                        case 2: stage_full<2>(st, hLaneS, yLaneS, hsrc, ysrc, pYStep, pYk, lane); break;
-                        case 4: stage_full<4>(st, hLaneS, yLaneS, hsrc, ysrc, pYStep, pYk, lane); break;
-                        case 8: stage_full<8>(st, hLaneS, yLaneS, hsrc, ysrc, pYStep, pYk, lane); break;
-                        default: stage_full<16>(st, hLaneS, yLaneS, hsrc, ysrc, pYStep, pYk, lane); break;
-                    }
-                } else {
-                    stage_item(p.cell[pci], phs, pys, pch, st, lane);
-                }
-            }
+            if (pch < pNFull)
+                stage_full<LTF>(st, hLaneS, yLaneS, phs + CHUNK * pch * LTF, pys + CHUNK * pch + pYLane, pYStep, pYk,
+                                lane);
+            else
+                stage_item_exact<LTF>(p.cell[pci], phs, pys, pch, st, lane);
             if (++pch == pNChunk) {
                 pch = 0;
                 if (++pq < pValid) {
@@ -1001,8 +976,7 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel(const __grid_constant_
     long grp = gw;
     int ci = 0;
     while (ci + 1 < p.nCells && grp >= p.cell[ci + 1].group0) ci++;
-    int q = 0, ch = 0, cslot = 0, nValid, cNChunk, cNFull, cA, cL, cLT, cHrs;
-    bool cExact = false;                                  // generic kernel: L fills the tile, aligned rows
+    int q = 0, ch = 0, cslot = 0, nValid, cNChunk, cNFull, cA;
     bool z2;
     uint32_t yo[2][2];
     unsigned long long ss = 0;                            // (scale, scale) of the cell's operands
@@ -1013,12 +987,8 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel(const __grid_constant_
         cA = cl.A;
         cNChunk = cl.nChunk;
         cNFull = cl.A / CHUNK;
-        cL = cl.L;
-        cLT = LTF != 0 ? LTF : cl.LT;
-        cHrs = cl.hrs;
-        cExact = cl.L == cl.LT && cl.LT >= 2 && cl.vecH && cl.vecY;
         z2 = cl.nSym > 8;
-        const uint32_t ys = CHUNK * (LTF != 0 ? hrs_of(LTF) : cl.hrs);
+        constexpr uint32_t ys = CHUNK * hrs_of(LTF);
 #pragma unroll
         for (int kk = 0; kk < 2; kk++)
 #pragma unroll
@@ -1048,42 +1018,13 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel(const __grid_constant_
         __syncwarp();                              // ... and every lane's
         const uint32_t st = stBase + cslot * p.stageBytes;
         cslot = cslot == NST - 1 ? 0 : cslot + 1;
-        if constexpr (LTF != 0) {
-            if (ch < cNFull)
-                mma_stage<LTF, P, true, true, SC>(st, hrs_of(LTF), CHUNK, LTF, yo, gacc, zacc, z2, g, c, ss);
-            else
-                mma_stage<LTF, P, true, false, SC>(st, hrs_of(LTF), cA - CHUNK * ch, LTF, yo, gacc, zacc, z2, g, c,
-                                                   ss);
-        } else {
-            const int nRows = min(CHUNK, cA - CHUNK * ch);
-            if (cExact && nRows == CHUNK) {
-                switch (cLT) {
-                    case 2: mma_stage<2, P, true, true, SC>(st, cHrs, CHUNK, 2, yo, gacc, zacc, z2, g, c, ss); break;
-                    case 4: mma_stage<4, P, true, true, SC>(st, cHrs, CHUNK, 4, yo, gacc, zacc, z2, g, c, ss); break;
-                    case 8: mma_stage<8, P, true, true, SC>(st, cHrs, CHUNK, 8, yo, gacc, zacc, z2, g, c, ss); break;
-                    default: mma_stage<16, P, true, true, SC>(st, cHrs, CHUNK, 16, yo, gacc, zacc, z2, g, c, ss); break;
-                }
-            } else switch (cLT) {
-                case 1: mma_stage<1, P, false, false, SC>(st, cHrs, nRows, cL, yo, gacc, zacc, z2, g, c, ss); break;
-                case 2: mma_stage<2, P, false, false, SC>(st, cHrs, nRows, cL, yo, gacc, zacc, z2, g, c, ss); break;
-                case 4: mma_stage<4, P, false, false, SC>(st, cHrs, nRows, cL, yo, gacc, zacc, z2, g, c, ss); break;
-                case 8: mma_stage<8, P, false, false, SC>(st, cHrs, nRows, cL, yo, gacc, zacc, z2, g, c, ss); break;
-                default: mma_stage<16, P, false, false, SC>(st, cHrs, nRows, cL, yo, gacc, zacc, z2, g, c, ss); break;
-            }
-        }
+        if (ch < cNFull)
+            mma_stage<LTF, P, true, SC>(st, hrs_of(LTF), CHUNK, yo, gacc, zacc, z2, g, c, ss);
+        else
+            mma_stage<LTF, P, false, SC>(st, hrs_of(LTF), cA - CHUNK * ch, yo, gacc, zacc, z2, g, c, ss);
         if (++ch < cNChunk) continue;
         ch = 0;
-        if constexpr (LTF != 0) {
-            store_acc<LTF>(sm, gacc, zacc, q, g, c);
-        } else {
-            switch (cLT) {
-                case 1: store_acc<1>(sm, gacc, zacc, q, g, c); break;
-                case 2: store_acc<2>(sm, gacc, zacc, q, g, c); break;
-                case 4: store_acc<4>(sm, gacc, zacc, q, g, c); break;
-                case 8: store_acc<8>(sm, gacc, zacc, q, g, c); break;
-                default: store_acc<16>(sm, gacc, zacc, q, g, c); break;
-            }
-        }
+        store_acc<LTF>(sm, gacc, zacc, q, g, c);
 #pragma unroll
         for (int b = 0; b < 3; b++)
 #pragma unroll
@@ -1100,23 +1041,167 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel(const __grid_constant_
             const FusedCell& cl = p.cell[ci];
             const CellView v = view_of(cl);
             const long sc0 = (grp - cl.group0) * cl.GS;
-            if constexpr (LTF != 0) {
-                solve_group<LTF, P>(v, sc0, nValid, smemOff, lane);
-            } else {
-                switch (cLT) {
-                    case 1: solve_group<1, P>(v, sc0, nValid, smemOff, lane); break;
-                    case 2: solve_group<2, P>(v, sc0, nValid, smemOff, lane); break;
-                    case 4: solve_group<4, P>(v, sc0, nValid, smemOff, lane); break;
-                    case 8: solve_group<8, P>(v, sc0, nValid, smemOff, lane); break;
-                    default: solve_group<16, P>(v, sc0, nValid, smemOff, lane); break;
-                }
-            }
+            solve_group<LTF, P>(v, sc0, nValid, smemOff, lane);
         }
         q = 0;
         grp += nw;
         if (grp >= total) break;
         while (ci + 1 < p.nCells && grp >= p.cell[ci + 1].group0) ci++;
         load_ccell();
+    }
+    cp_async_wait<0>();
+}
+
+// ---------------------------------------------------------------------------
+// Any mix of cells.  A warp takes a group at a time through the code of its
+// cell's layer tile: the tile is chosen once per group and the chunk loop
+// inside knows it at compile time.  (Choosing it for every chunk, once to copy
+// and once to multiply, with a copy cursor that could change cell at any
+// chunk, spent most of the instructions of such a launch on that.)  The copies
+// of the next chunk are always one ahead, at a group's end those of the warp's
+// next group's first chunk.  Kernel times with the cursor and per-chunk masks
+// and divisions -> as here: the uneven 16-cell batch 33.0 -> 30.1 us, 12 ragged
+// cells 28.7 -> 21.6 us, 24 of them 42.7 -> 25.0 us (of which the last two owe
+// part to the copies without divisions, stage_any).
+// ---------------------------------------------------------------------------
+struct MixedWarp {
+    uint32_t stBase;                   // first operand stage
+    int lane, g, c, slot;              // slot: the stage of the item at hand
+};
+
+// First chunk of group grp of cell cl into the stage at st.
+__device__ __noinline__ void stage_first(const FusedCell& cl, long grp, uint32_t st, int lane) {
+    const long sc = (grp - cl.group0) * cl.GS;
+    stage_any(cl, cl.H + sc * cl.A * cl.L, cl.Y + sc * cl.nSym * cl.A, min(CHUNK, cl.A), st, lane);
+}
+
+// The items of one group, G and Z of its subcarriers into sm, then the solve.
+// EX: the cell's layers fill the tile LT, its antennas whole chunks, and its
+// rows are 16-byte aligned.  ng / nci: the warp's next group (ng >= total: none).
+template <int LT, bool EX, int P, bool SC>
+__device__ __forceinline__ void run_group(const FusedParams& p, MixedWarp& w, int ci, long grp, int nci, long ng,
+                                          float2* sm, int smemOff) {
+    const FusedCell& cl = p.cell[ci];
+    const int A = cl.A, L = EX ? LT : cl.L, nSym = cl.nSym, nChunk = cl.nChunk;
+    const int hrs = EX ? hrs_of(LT) : cl.hrs;
+    const int nValid = group_valid(cl, grp);
+    const long sc0 = (grp - cl.group0) * cl.GS;
+    const bool z2 = nSym > 8;
+    unsigned long long ss = 0;
+    if constexpr (SC) ss = pk2(cl.scale, cl.scale);
+    uint32_t yo[2][2];
+#pragma unroll
+    for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++) {
+            const int r = 8 * nt + w.g;
+            const int ra = r < nSym ? r : 0;             // rows past nSym are not staged: read row 0 instead
+            yo[kk][nt] = CHUNK * hrs + ra * 128 + (((4 * kk + w.c) ^ ((ra & 1) << 2)) << 4);
+        }
+    // the next item's channel run and received rows
+    const float2* hs = cl.H + sc0 * A * L;
+    const float2* ys = cl.Y + sc0 * nSym * A;
+    // EX: this lane's stage offsets, first received piece and count of rows
+    uint32_t hLaneS = 0, yLaneS = 0;
+    int yLane = 0, yk = 0;
+    if constexpr (EX) {
+        constexpr int HALF = LT / 2;
+        hLaneS = (w.lane / HALF) * hrs_of(LT) + (w.lane % HALF) * 16;
+        yLaneS = CHUNK * hrs_of(LT) + (w.lane >> 3) * 128 + (((w.lane & 7) ^ (((w.lane >> 3) & 1) << 2)) << 4);
+        yLane = (w.lane >> 3) * A + 2 * (w.lane & 7);
+        yk = min(4, max(0, (nSym - (w.lane >> 3) + 3) >> 2));
+    }
+    float gacc[3][4], zacc[2][2][4];
+    for (int q = 0; q < nValid; q++) {
+#pragma unroll
+        for (int b = 0; b < 3; b++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) gacc[b][e] = 0.f;
+#pragma unroll
+        for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+            for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) zacc[mt][nt][e] = 0.f;
+#pragma unroll 1
+        for (int ch = 0; ch < nChunk; ch++) {
+            __syncwarp();                              // every lane is done with the stage refilled now
+            const uint32_t st = w.stBase + w.slot * p.stageBytes;
+            const uint32_t next = w.stBase + (w.slot ^ 1) * p.stageBytes;
+            w.slot ^= 1;
+            int nch = ch + 1;
+            bool more = true;                          // the next item is this group's too
+            if (nch == nChunk) {
+                nch = 0;
+                more = q + 1 < nValid;
+                hs += (long)A * L;
+                ys += (long)nSym * A;
+            }
+            if (more) {
+                if constexpr (EX)
+                    stage_full<LT>(next, hLaneS, yLaneS, hs + CHUNK * nch * LT, ys + CHUNK * nch + yLane, 4 * A, yk,
+                                   w.lane);
+                else
+                    stage_any(cl, hs + CHUNK * nch * L, ys + CHUNK * nch, min(CHUNK, A - CHUNK * nch), next, w.lane);
+            } else if (ng < p.totalGroups) {
+                stage_first(p.cell[nci], ng, next, w.lane);
+            }
+            cp_async_commit();
+            cp_async_wait<1>();                        // this item's copies (own lane) have landed
+            __syncwarp();                              // ... and every lane's
+            mma_stage<LT, P, EX, SC>(st, hrs, A - CHUNK * ch, yo, gacc, zacc, z2, w.g, w.c, ss);
+        }
+        store_acc<LT>(sm, gacc, zacc, q, w.g, w.c, L);
+    }
+    __syncwarp();
+    solve_group<LT, P, false, true>(view_of(cl), sc0, nValid, smemOff, w.lane);
+}
+
+template <int P, bool SC = false>
+__global__ void __launch_bounds__(256, 2) fused_eq_kernel_m(const __grid_constant__ FusedParams p) {
+    extern __shared__ float4 smem_raw[];
+    const int wib = threadIdx.x >> 5;
+    const int warpsPerCta = blockDim.x >> 5;
+    const int warpBytes = p.epiBytes + stages_of(0) * p.stageBytes;
+    const int smemOff = wib * (warpBytes / 8);
+    float2* sm = reinterpret_cast<float2*>(smem_raw) + smemOff;
+    MixedWarp w;
+    w.lane = threadIdx.x & 31;
+    w.g = w.lane >> 2;
+    w.c = w.lane & 3;
+    w.slot = 0;
+    w.stBase =
+        (uint32_t)__cvta_generic_to_shared(reinterpret_cast<char*>(smem_raw) + (long)wib * warpBytes + p.epiBytes);
+    const long nw = (long)gridDim.x * warpsPerCta;
+    long grp = (long)blockIdx.x * warpsPerCta + wib;
+    if (grp >= p.totalGroups) return;
+    static_assert(stages_of(0) == 2, "one item ahead");
+    int ci = 0;
+    while (ci + 1 < p.nCells && grp >= p.cell[ci + 1].group0) ci++;
+    stage_first(p.cell[ci], grp, w.stBase, w.lane);
+    cp_async_commit();
+    while (grp < p.totalGroups) {
+        const long ng = grp + nw;
+        int nci = ci;
+        while (nci + 1 < p.nCells && ng >= p.cell[nci + 1].group0) nci++;
+        if (p.cell[ci].exact) {
+            switch (p.cell[ci].LT) {
+                case 2: run_group<2, true, P, SC>(p, w, ci, grp, nci, ng, sm, smemOff); break;
+                case 4: run_group<4, true, P, SC>(p, w, ci, grp, nci, ng, sm, smemOff); break;
+                case 8: run_group<8, true, P, SC>(p, w, ci, grp, nci, ng, sm, smemOff); break;
+                default: run_group<16, true, P, SC>(p, w, ci, grp, nci, ng, sm, smemOff); break;
+            }
+        } else {
+            switch (p.cell[ci].LT) {
+                case 1: run_group<1, false, P, SC>(p, w, ci, grp, nci, ng, sm, smemOff); break;
+                case 2: run_group<2, false, P, SC>(p, w, ci, grp, nci, ng, sm, smemOff); break;
+                case 4: run_group<4, false, P, SC>(p, w, ci, grp, nci, ng, sm, smemOff); break;
+                case 8: run_group<8, false, P, SC>(p, w, ci, grp, nci, ng, sm, smemOff); break;
+                default: run_group<16, false, P, SC>(p, w, ci, grp, nci, ng, sm, smemOff); break;
+            }
+        }
+        grp = ng;
+        ci = nci;
     }
     cp_async_wait<0>();
 }
@@ -1286,8 +1371,7 @@ __global__ void __launch_bounds__(256, LTF == 16 ? 1 : 2) fused_eq_kernel_a(cons
             pslot = pslot == NST - 1 ? 0 : pslot + 1;
             cp_async_wait<NST - 1>();                  // this chunk's copies (own lane) have landed
             __syncwarp();                              // ... and every lane's
-            mma_stage<LTF, P, true, true, SC>(stBase + cslot * p.stageBytes, HRS, CHUNK, LTF, yo, gacc, zacc, z2, g,
-                                              c, ss);
+            mma_stage<LTF, P, true, SC>(stBase + cslot * p.stageBytes, HRS, CHUNK, yo, gacc, zacc, z2, g, c, ss);
             cslot = cslot == NST - 1 ? 0 : cslot + 1;
         }
         store_acc<LTF>(sm, gacc, zacc, q, g, c);
@@ -1840,11 +1924,13 @@ int build_fused_params(const aerial_cell_desc* cells, int nCells, FusedParams& p
         f.vecH = ((c.nLayers % 2) == 0 && ((uintptr_t)c.H & 15) == 0) ? 1 : 0;
         {
             const int half = c.nLayers / 2;
-            f.lgHalfL = (half > 0 && (half & (half - 1)) == 0) ? __builtin_ctz(half) : -1;
+            f.lgHalfL = (half > 0 && (half & (half - 1)) == 0) ? __builtin_ctz(half) : 0;
         }
         f.lut = pam_lut(c.nPamBits);
         f.nChunk = (c.nAnt + CHUNK - 1) / CHUNK;
-        f.hrs = hrs_of(c.nLayers);
+        f.hrs = hrs_any(c.nLayers);
+        f.vecRun = ((c.nAnt * c.nLayers) % 2) == 0 && ((uintptr_t)c.H & 15) == 0;
+        f.exact = f.LT >= 2 && f.L == f.LT && f.vecH && f.vecY && c.nAnt % CHUNK == 0;
         // LLR rows of 2*nPam floats are written as float4 for nPam 2/4: need 16 B alignment
         if ((c.nPamBits == 2 || c.nPamBits == 4) && ((uintptr_t)c.llr & 15)) return AERIAL_ERR_INVALID_ARG;
     }
@@ -2064,8 +2150,12 @@ static int plan_p(const FusedParams& p, int warpBytes, LaunchShape sh, LaunchPla
         case 4: return plan_v<P, 4, SC>(p, warpBytes, sh, out);
         case 8: return plan_v<P, 8, SC>(p, warpBytes, sh, out);
         case 16: return plan_v<P, 16, SC>(p, warpBytes, sh, out);
-        default: return plan_v<P, 0, SC>(p, warpBytes, sh, out);
+        default: break;
     }
+    const int s = allow_max_smem<fused_eq_kernel_m<P, SC>>();
+    if (s) return s;
+    fill_plan(reinterpret_cast<const void*>(fused_eq_kernel_m<P, SC>), p, warpBytes, sh, out);
+    return AERIAL_OK;
 }
 
 int plan_fused(const FusedParams& p, int warpBytes, int prec, LaunchShape sh, LaunchPlan& out) {
@@ -2530,7 +2620,11 @@ static int prepare_p() {
     if (!s) s = prepare_an<P, 4, SC>();
     if (!s) s = prepare_an<P, 8, SC>();
     if (!s) s = prepare_an<P, 16, SC>();
-    if (!s) s = prepare_v<P, 0, SC>();
+    if (!s) {
+        cudaFuncAttributes at;
+        const cudaError_t e = cudaFuncGetAttributes(&at, fused_eq_kernel_m<P, SC>);
+        s = e == cudaSuccess ? allow_max_smem<fused_eq_kernel_m<P, SC>>() : rt_status(e);
+    }
     if (!s) s = prepare_v<P, 2, SC>();
     if (!s) s = prepare_v<P, 4, SC>();
     if (!s) s = prepare_v<P, 8, SC>();
