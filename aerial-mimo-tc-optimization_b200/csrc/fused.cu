@@ -28,6 +28,7 @@
 // covers antennas 8j+2c and 8j+2c+1 of k-step j (the K order is permuted
 // inside each k-step; A and B use the same permutation).
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -338,7 +339,11 @@ __device__ __forceinline__ float4 lds128(uint32_t a) {
 // raw FP16 is safe are multiplied by the cell's power-of-two scale ss = (s, s)
 // before they are rounded (exact; the cell's sigma2 carries s^2, so G^-1 Z,
 // mu and the LLRs are unchanged).
-template <int LT, int P, bool FULL, bool SC = false>
+// NZ: symbol tiles of 8 (1 or 2), or 0 where z2 says at run time; known, the
+// whole chunk is one block of straight code, whose loads the compiler moves
+// ahead of the products (12-slot precision-stress launch with BF16X3 operands
+// 303 -> 294 us, 64 100 MHz slots 208 -> 207 us, complex half 141 -> 138 us).
+template <int LT, int P, bool FULL, bool SC = false, int NZ = 0>
 __device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, const uint32_t (&yo)[2][2],
                                           float (*gacc)[4], float (*zacc)[2][4], bool z2, int g, int c,
                                           unsigned long long ss = 0) {
@@ -357,12 +362,14 @@ __device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, const
         }
         float4 yv[2];
 #pragma unroll
-        for (int nt = 0; nt < 2; nt++) yv[nt] = lds128(st + yo[kk][nt]);
+        for (int nt = 0; nt < 2; nt++)
+            if (NZ != 1 || nt == 0) yv[nt] = lds128(st + yo[kk][nt]);
         if constexpr (SC) {
 #pragma unroll
             for (int mt = 0; mt < NMT; mt++) hv[mt] = scale4(hv[mt], ss);
 #pragma unroll
-            for (int nt = 0; nt < 2; nt++) yv[nt] = scale4(yv[nt], ss);
+            for (int nt = 0; nt < 2; nt++)
+                if (NZ != 1 || nt == 0) yv[nt] = scale4(yv[nt], ss);
         }
         if constexpr (P == AERIAL_PREC_BF16X3 || P == AERIAL_PREC_FP16X3) {
             uint32_t ah[NMT][2], al[NMT][2];
@@ -374,6 +381,7 @@ __device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, const
             uint32_t yh[2][2], yl[2][2];
 #pragma unroll
             for (int nt = 0; nt < 2; nt++) {
+                if (NZ == 1 && nt == 1) break;
                 split2<P>(yv[nt].x, yv[nt].y, yh[nt][0], yl[nt][0]);
                 split2<P>(yv[nt].z, yv[nt].w, yh[nt][1], yl[nt][1]);
             }
@@ -390,7 +398,7 @@ __device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, const
                 }
 #pragma unroll
                 for (int nt = 0; nt < 2; nt++) {
-                    if (nt == 1 && !z2) break;
+                    if (nt == 1 && (NZ == 1 || (NZ == 0 && !z2))) break;
                     mma16816<P>(zacc[mt][nt], h0, h1, h2, h3, yh[nt][0], yh[nt][1]);
                     mma16816<P>(zacc[mt][nt], h0, h1, h2, h3, yl[nt][0], yl[nt][1]);
                     mma16816<P>(zacc[mt][nt], l0, l1, l2, l3, yh[nt][0], yh[nt][1]);
@@ -406,6 +414,7 @@ __device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, const
             uint32_t b[2][2];
 #pragma unroll
             for (int nt = 0; nt < 2; nt++) {
+                if (NZ == 1 && nt == 1) break;
                 b[nt][0] = pack2<P>(yv[nt].x, yv[nt].y);
                 b[nt][1] = pack2<P>(yv[nt].z, yv[nt].w);
             }
@@ -416,7 +425,7 @@ __device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, const
                 for (int nt = 0; nt <= mt; nt++) mma16816<P>(gacc[mt + nt], a0r, a1r, a2r, a3r, a[nt][0], a[nt][1]);
 #pragma unroll
                 for (int nt = 0; nt < 2; nt++) {
-                    if (nt == 1 && !z2) break;
+                    if (nt == 1 && (NZ == 1 || (NZ == 0 && !z2))) break;
                     mma16816<P>(zacc[mt][nt], a0r, a1r, a2r, a3r, b[nt][0], b[nt][1]);
                 }
             }
@@ -1359,6 +1368,7 @@ __global__ void __launch_bounds__(256, LTF == 16 ? 1 : 2) fused_eq_kernel_a(cons
         // by 2 299.5 / 238.0, not unrolled 293-295 / 240 us.  The 8-layer
         // tile with 128 antennas (8 chunks) is unrolled by 4: 16 cells of
         // 106 PRB, BF16X3 94.7-96.6 -> 92.6-92.8 us (FP16 88.5 us either way).
+        auto chunks = [&](auto nz) {
 #pragma unroll(LTF == 16 ? 1 : (LTF == 8 && NCH == 8 ? 4 : NCH))
         for (int k = 0; k < NCH; k++) {
             __syncwarp();                              // every lane is done with the slot refilled now
@@ -1371,9 +1381,12 @@ __global__ void __launch_bounds__(256, LTF == 16 ? 1 : 2) fused_eq_kernel_a(cons
             pslot = pslot == NST - 1 ? 0 : pslot + 1;
             cp_async_wait<NST - 1>();                  // this chunk's copies (own lane) have landed
             __syncwarp();                              // ... and every lane's
-            mma_stage<LTF, P, true, SC>(stBase + cslot * p.stageBytes, HRS, CHUNK, yo, gacc, zacc, z2, g, c, ss);
+            mma_stage<LTF, P, true, SC, nz.value>(stBase + cslot * p.stageBytes, HRS, CHUNK, yo, gacc, zacc, z2, g, c, ss);
             cslot = cslot == NST - 1 ? 0 : cslot + 1;
         }
+        };
+        if (z2) chunks(std::integral_constant<int, 2>{});
+        else chunks(std::integral_constant<int, 1>{});
         store_acc<LTF>(sm, gacc, zacc, q, g, c);
         cur = nxt;
         if (++q < nValid) continue;
@@ -1441,9 +1454,10 @@ __device__ __forceinline__ uint2 lds64u(uint32_t a) {
 // 16 layers: two m-tiles (layers g and g + 8, 32 bytes apart in a row), the
 // Gram blocks (0,0), (1,0), (1,1) and both matched-filter m-tiles, each
 // accumulator fed in the complex64 kernel's order (mma_stage).
-template <int LT>
+template <int LT, int NZ = 0>
 __device__ __forceinline__ void mma_stage_h(uint32_t st, uint32_t hb, const uint32_t (&yo)[2][2],
                                             float (*gacc)[4], float (*zacc)[2][4], bool z2) {
+    if constexpr (NZ != 0) z2 = NZ == 2;
     constexpr int HRS = hrs16_of(LT);
 #pragma unroll
     for (int kk = 0; kk < 2; kk++) {
@@ -1573,6 +1587,7 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel_h(const __grid_constan
         // 16 layers: unrolled by 2 for the instruction cache (the 12-slot
         // complex-half precision-stress launch 180.7 -> 174.6 us, same box,
         // bit-identical)
+        auto chunks = [&](auto nz) {
 #pragma unroll(LTF == 16 ? 2 : NCH)
         for (int k = 0; k < NCH; k++) {
             __syncwarp();                              // every lane is done with the slot refilled now
@@ -1586,9 +1601,12 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel_h(const __grid_constan
             cp_async_wait<NST - 1>();                  // this chunk's copies (own lane) have landed
             __syncwarp();                              // ... and every lane's
             const uint32_t st = stBase + cslot * p.stageBytes;
-            mma_stage_h<LTF>(st, st + hoff, yo, gacc, zacc, z2);
+            mma_stage_h<LTF, nz.value>(st, st + hoff, yo, gacc, zacc, z2);
             cslot = cslot == NST - 1 ? 0 : cslot + 1;
         }
+        };
+        if (z2) chunks(std::integral_constant<int, 2>{});
+        else chunks(std::integral_constant<int, 1>{});
         store_acc<LTF>(sm, gacc, zacc, q, g, c);
         cur = nxt;
         if (++q < nValid) continue;
