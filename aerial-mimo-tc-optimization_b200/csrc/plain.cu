@@ -10,32 +10,39 @@
 namespace aeq {
 
 // ---------------------------------------------------------------------------
-// One kernel for the solve, the apply and the whole chain.  A team of TEAM
-// lanes owns a subcarrier; its H, Y and C sit in shared memory, G and the
-// trailing block of the factor in registers.
+// One kernel for the solve, the apply and the whole chain.  A block takes
+// several subcarriers, a team of TEAM lanes each, with their H, then Y, and C in
+// shared memory.
 //
 //   kCoef   G, H -> C, noiseInv          the FP32 Cholesky MMSE solve
 //   kApply  C, Y -> Y_eq                 coef_apply_v1_scalar (src/aerial_coef_wmma.cu:71-104)
-//   kChain  H, Y -> LLR (and Y_eq)       all of them and the demapper; G, C and noiseInv
-//                                        never leave the SM
+//   kChain  H, Y -> LLR (and Y_eq)       gram_scalar (src/aerial_bottleneck.cu:56-80, M = H^H),
+//                                        all of the above and the demapper; G, C and
+//                                        noiseInv never leave the SM
 //
 // Every value is accumulated in the serial specification's order with its
 // fused multiply-adds; lanes only divide the values among themselves:
-//   G       lane: row r, columns 2p, 2p + 1, antennas in order.
-//   factor  column by column, right-looking: the lane that holds (i, j) takes
-//           L_ik conj(L_jk) off it at step k = 0, 1, ..., which is the order
-//           of the left-looking sum.
+//   G       lane: row r, columns 2q, 2q + 1, antennas in order.
+//   factor  right-looking, lane: row i: at step k = 0, 1, ... it takes
+//           L_ik conj(L_jk) off its element j, the order of the left-looking sum.
 //   C       lane: antennas tid, tid + TEAM, ... (two at a time, for two
 //           independent chains); forward and backward substitution in registers.
-//   mu      lane l: sum over the antennas in order.
+//   mu      lane: one layer, antennas in order.
 //   Y_eq    lane: one layer and up to TS symbols, antennas in order.
 //
-// What bounds it: the FMA and shared-memory pipes at about equal shares.  A
-// thread per output element, as the reference has it, reads two operands from
-// L1 for each complex product; here a lane's operands serve two columns (G)
-// or up to four symbols (Y_eq) from one 16-byte read each, rows are padded so
-// that a warp's reads meet no bank conflicts, and the intermediates' 27.6 MB
-// per 100 MHz slot of HBM traffic are gone from the chain.
+// What bounds it: instruction issue and the latency of each subcarrier's chain
+// of phases.  A thread per output element, as the reference has it, reads two
+// operands from L1 for each complex product; here a lane's operands serve two
+// columns (G) or up to four symbols (Y_eq) from one 16-byte read each, rows are
+// padded so that a warp's reads meet no bank conflicts, and the intermediates'
+// 27.6 MB per 100 MHz slot of HBM traffic are gone.  The phases with fewer
+// values than lanes (the factor, with its square roots and divisions, and mu)
+// run for all subcarriers of a block in one warp: done by each subcarrier's own
+// warp they were over a quarter of all instructions.  Y is copied where H was
+// once H is spent (and asked into L2 at the start), which leaves room for 20
+// subcarriers on an SM instead of 12.  4 slots of 132 PRB x 64 antennas x 8
+// layers: 403 us as four scalar kernels per cell, 53 us with a warp for each
+// subcarrier throughout, 48 us as here.
 // ---------------------------------------------------------------------------
 enum PlainMode : int { kCoef, kApply, kChain };
 
@@ -56,26 +63,33 @@ struct PlainCell {
 struct PlainParams {
     PlainCell cell[AERIAL_MAX_CELLS];
     int nCells;
-    int teamBytes;      // shared memory per team
+    int teamValues;     // shared memory per team, in complex values (even)
 };
 
 // Lanes per subcarrier: 16 for up to 4 layers, a warp for 8, four warps for
-// 16 (whose factor has 72 column pairs and whose C needs 128 antennas' worth
-// of lanes to keep the FMA pipe fed at two or three resident blocks per SM).
+// 16, whose C has enough antennas to occupy them.  A block's subcarriers have at
+// most 32 rows between them (the factor's warp).
 __host__ __device__ constexpr int plain_team(int LT) { return LT <= 4 ? 16 : LT == 8 ? 32 : 128; }
+constexpr int kPlainThreads = 128;
 
 // Row strides in complex values: even (16-byte rows) and 16 bytes past a
 // multiple of the row, so that eight rows read at once differ in banks.
 __host__ __device__ __forceinline__ int plain_hs(int L) { return ((L + 1) & ~1) + 2; }
 __host__ __device__ __forceinline__ int plain_cs(int A) { return ((A + 1) & ~1) + 2; }
 
-static int plain_team_bytes(int mode, int A, int L, int S) {
-    int v = 0;
-    if (mode != kApply) v += A * plain_hs(L);
-    v += L * plain_cs(A);
-    if (mode != kCoef) v += S * plain_cs(A);
-    if (mode != kApply) v += L * L + ((3 * L + 1) / 2 + 1);
-    return ((v + 1) & ~1) * (int)sizeof(cf);
+// Shared memory of a team, in complex values: H (kChain: then Y), C, Y (kApply),
+// G and then the factor, and 3 L floats.
+struct PlainSmem {
+    int c, y, l, total;
+};
+__host__ __device__ __forceinline__ PlainSmem plain_smem(int mode, int A, int L, int S) {
+    const int h = A * plain_hs(L), c = L * plain_cs(A), y = S * plain_cs(A);
+    PlainSmem m;
+    m.c = mode == kApply ? 0 : mode == kCoef ? h : (h > y ? h : y);
+    m.y = mode == kApply ? c : 0;
+    m.l = m.c + c + (mode == kApply ? y : 0);
+    m.total = (m.l + (mode == kApply ? 0 : L * L + (3 * L + 1) / 2) + 1) & ~1;
+    return m;
 }
 
 template <int TEAM>
@@ -212,7 +226,7 @@ __device__ __forceinline__ void apply_symbols(const PlainCell& cl, const cf* sC,
         acc[t] = make_float2(0.f, 0.f);
     }
     int a = 0;
-#pragma unroll 2
+#pragma unroll 4
     for (; a + 1 < A; a += 2) {
         const float4 cv = ld4(c + a);
         float4 yv[TS];
@@ -245,120 +259,152 @@ __device__ __forceinline__ void apply_symbols(const PlainCell& cl, const cf* sC,
     }
 }
 
+// Cholesky factor of the block's subcarriers by one warp, lane (j, i) = row i of
+// subcarrier j: G's lower triangle at sl (row stride L, next subcarrier ts
+// later) is replaced by the factor's, 1 / its diagonal goes to sInv.
+template <int LT, bool EX>
+__device__ __forceinline__ void factor_rows(cf* sl, float* sInv, int L, int i) {
+    cf r[LT];
+#pragma unroll
+    for (int c = 0; c < LT; c++) r[c] = (c <= i && i < L) ? sl[i * L + c] : make_float2(1.f, 0.f);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < LT; k++) {
+        if (!EX && k >= L) break;
+        float s = __shfl_sync(0xffffffffu, r[k].x, k, LT);
+        if (!(s > 0.f)) s = 1e-30f;
+        const float iv = __fdiv_rn(1.0f, __fsqrt_rn(s));
+        if (i == k) sInv[k] = iv;
+        const cf a = make_float2(__fmul_rn(r[k].x, iv), __fmul_rn(r[k].y, iv));
+        if (i > k && i < L) sl[i * L + k] = a;
+        __syncwarp();
+#pragma unroll
+        for (int c = k + 1; c < LT; c++) {
+            if (!EX && c >= L) break;
+            const cf b = sl[c * L + k];
+            r[c].x = __fmaf_rn(-a.x, b.x, r[c].x);
+            r[c].x = __fmaf_rn(-a.y, b.y, r[c].x);
+            r[c].y = __fmaf_rn(-a.y, b.x, r[c].y);
+            r[c].y = __fmaf_rn(a.x, b.y, r[c].y);
+        }
+    }
+}
+
 // EX: every cell has L == LT.  LT: layers rounded up to 2, 4, 8 or 16.
 template <int MODE, int LT, bool EX>
-__global__ void __launch_bounds__(128) plain_kernel(const __grid_constant__ PlainParams p) {
+__global__ void __launch_bounds__(kPlainThreads) plain_kernel(const __grid_constant__ PlainParams p) {
     constexpr int TEAM = plain_team(LT);
     constexpr int LPL = TEAM / LT;                     // lanes per layer of the apply phase
-    extern __shared__ float4 plain_smem[];
-    const int team = threadIdx.x / TEAM, tid = threadIdx.x % TEAM;
+    extern __shared__ float4 plain_shared[];
+    const int team = threadIdx.x / TEAM, tid = threadIdx.x % TEAM, teams = blockDim.x / TEAM;
     int ci = 0;
     while (ci + 1 < p.nCells && blockIdx.x >= p.cell[ci + 1].block0) ci++;
     const PlainCell& cl = p.cell[ci];
     const int A = cl.A, L = EX ? LT : cl.L, S = cl.S;
     const int hs = EX ? LT + 2 : plain_hs(L), cs = plain_cs(A);
-    const long scw = (long)(blockIdx.x - cl.block0) * (blockDim.x / TEAM) + team;
-    const bool out = scw < cl.nSC;                     // teams past the cell's end repeat its last subcarrier
-    const long sc = out ? scw : cl.nSC - 1;
-    cf* sH = reinterpret_cast<cf*>(reinterpret_cast<char*>(plain_smem) + (size_t)team * p.teamBytes);
-    cf* sC = sH + (MODE != kApply ? A * hs : 0);
-    cf* sY = sC + L * cs;
-    cf* sL = sY + (MODE != kCoef ? S * cs : 0);
-    float* sInv = reinterpret_cast<float*>(sL + L * L);
-    float* sMuInv = sInv + L;
-    float* sNoise = sMuInv + L;
+    const long sc0 = (long)(blockIdx.x - cl.block0) * teams;
+    const bool out = sc0 + team < cl.nSC;              // teams past the cell's end repeat its last subcarrier
+    const long sc = out ? sc0 + team : cl.nSC - 1;
+    const int ts = p.teamValues;
+    const PlainSmem m = plain_smem(MODE, A, L, S);
+    cf* sh = reinterpret_cast<cf*>(plain_shared);      // team 0's
+    cf* sH = sh + team * ts;
+    cf* sC = sH + m.c;
+    cf* sY = sH + m.y;
 
-    if constexpr (MODE != kApply) stage_rows<TEAM, EX ? LT : 0>(sH, hs, cl.H + sc * A * L, A, L, cl.vecH, tid);
-    else stage_rows<TEAM>(sC, cs, cl.C + sc * A * L, L, A, cl.vecY, tid);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    if constexpr (MODE != kCoef)
+    if constexpr (MODE == kApply) {
+        stage_rows<TEAM>(sC, cs, cl.C + sc * A * L, L, A, cl.vecY, tid);
         stage_rows<TEAM>(sY, cs, cl.Y + sc * S * A, S, A, cl.vecY, tid);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    team_sync<TEAM>();
+    } else {
+        stage_rows<TEAM, EX ? LT : 0>(sH, hs, cl.H + sc * A * L, A, L, cl.vecH, tid);
+        if constexpr (MODE == kChain) {
+            const char* y = reinterpret_cast<const char*>(cl.Y + sc * S * A);
+            for (int e = 128 * tid; e < 8 * S * A; e += 128 * TEAM)
+                asm volatile("prefetch.global.L2 [%0];\n" ::"l"(__cvta_generic_to_global(y + e)));
+        } else {
+            for (int e = tid; e < L * L; e += TEAM) sH[m.l + e] = cl.G[sc * L * L + e];
+        }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 
     float noise = 0.f;
     if constexpr (MODE != kApply) {
-        // the lower triangle: row pair R holds 2 (R + 1) column pairs, after
-        // the R (R + 1) of the pairs above
-        int R = 0;
-        while ((R + 1) * (R + 2) <= tid) R++;
-        const int u = tid - R * (R + 1);
-        const int r = 2 * R + (u > R ? 1 : 0), q = u > R ? u - R - 1 : u;
-        const bool own = r < L;
-        cf g0 = make_float2(0.f, 0.f), g1 = g0;        // (r, 2q), (r, 2q + 1)
-        if (own) {
-            if constexpr (MODE == kChain) {
-                const cf* hr = sH + r;
-                const cf* hc = sH + 2 * q;
-#pragma unroll 4
+        __syncthreads();
+        if constexpr (MODE == kChain) {
+            // the lower triangle of G: row pair R holds 2 (R + 1) column pairs,
+            // after the R (R + 1) of the pairs above
+            constexpr int PAIRS = LT / 2 * (LT / 2 + 1);
+            for (int t = threadIdx.x; t < teams * PAIRS; t += blockDim.x) {
+                const int j = t / PAIRS, v = t % PAIRS;
+                int R = 0;
+                while ((R + 1) * (R + 2) <= v) R++;
+                const int u = v - R * (R + 1);
+                const int r = 2 * R + (u > R ? 1 : 0), q = u > R ? u - R - 1 : u;
+                if (!EX && r >= L) continue;
+                const cf* hr = sh + j * ts + r;
+                const cf* hc = sh + j * ts + 2 * q;
+                cf g0 = make_float2(0.f, 0.f), g1 = g0;
+#pragma unroll 8
                 for (int k = 0; k < A; k++) {
-                    const cf v = hr[k * hs];
+                    const cf w = hr[k * hs];
                     const float4 c = ld4(hc + k * hs);
-                    const cf m = make_float2(v.x, -v.y);
-                    g0 = cma(m, make_float2(c.x, c.y), g0);
-                    g1 = cma(m, make_float2(c.z, c.w), g1);
+                    const cf n = make_float2(w.x, -w.y);
+                    g0 = cma(n, make_float2(c.x, c.y), g0);
+                    g1 = cma(n, make_float2(c.z, c.w), g1);
                 }
                 if (r == 2 * q) g0.x = __fadd_rn(g0.x, cl.sigma2);
                 if (r == 2 * q + 1) g1.x = __fadd_rn(g1.x, cl.sigma2);
-            } else {
-                const cf* g = cl.G + (sc * L + r) * L + 2 * q;
-                g0 = g[0];
-                if (2 * q + 1 <= r) g1 = g[1];
+                cf* g = sh + j * ts + m.l + r * L + 2 * q;
+                g[0] = g0;
+                if (2 * q + 1 <= r) g[1] = g1;
             }
+            __syncthreads();
         }
-        for (int k = 0; k < L; k++) {
-            const bool odd = k & 1;
-            if (own && q == (k >> 1)) {
-                cf& e = odd ? g1 : g0;
-                if (r == k) {
-                    float s = e.x;
-                    if (!(s > 0.f)) s = 1e-30f;
-                    sInv[k] = __fdiv_rn(1.0f, __fsqrt_rn(s));
-                }
-            }
-            team_sync<TEAM>();
-            if (own && q == (k >> 1) && r > k) {
-                const cf e = odd ? g1 : g0;
-                const float iv = sInv[k];
-                sL[r * L + k] = make_float2(__fmul_rn(e.x, iv), __fmul_rn(e.y, iv));
-            }
-            team_sync<TEAM>();
-            if (own && 2 * q + 1 > k && r > k) {
-                const cf a = sL[r * L + k];
-                auto take = [&](cf b, cf& e) {
-                    e.x = __fmaf_rn(-a.x, b.x, e.x);
-                    e.x = __fmaf_rn(-a.y, b.y, e.x);
-                    e.y = __fmaf_rn(-a.y, b.x, e.y);
-                    e.y = __fmaf_rn(a.x, b.y, e.y);
-                };
-                if (2 * q > k) take(sL[2 * q * L + k], g0);
-                if (2 * q + 1 <= r) take(sL[(2 * q + 1) * L + k], g1);
-            }
+        // one warp, another one from block to block
+        const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+        const bool mine = (int)(threadIdx.x >> 5) == (int)(blockIdx.x % (unsigned)warps);
+        if (mine) {
+            const int j = min(lane / LT, teams - 1);   // lanes past the last subcarrier repeat it
+            cf* l = sh + j * ts + m.l;
+            factor_rows<LT, EX>(l, reinterpret_cast<float*>(l + L * L), L, lane % LT);
         }
+        __syncthreads();
         // ---- C: forward and backward substitution per antenna ----
+        const cf* sL = sH + m.l;
+        const float* sInv = reinterpret_cast<const float*>(sL + L * L);
         int a = tid;
         for (; a + TEAM < A; a += 2 * TEAM) solve_antennas<LT, EX, 2, TEAM>(sH, hs, sL, sInv, sC, cs, L, a);
         if (a < A) solve_antennas<LT, EX, 1, TEAM>(sH, hs, sL, sInv, sC, cs, L, a);
-        team_sync<TEAM>();
+        __syncthreads();
         // ---- mu and the noise of the unbiased symbol ----
-        if (tid < L) {
-            float mu = 0.f;
-            const cf* c = sC + tid * cs;
-            const cf* h = sH + tid;
+        if (mine) {
+            const int j = lane / LT, l = lane % LT;
+            if (j < teams && l < L) {
+                float mu = 0.f;
+                const cf* c = sh + j * ts + m.c + l * cs;
+                const cf* h = sh + j * ts + l;
 #pragma unroll 8
-            for (int k = 0; k < A; k++) {
-                const cf cv = c[k], hv = h[k * hs];
-                mu = __fmaf_rn(cv.x, hv.x, mu);
-                mu = __fmaf_rn(-cv.y, hv.y, mu);
+                for (int k = 0; k < A; k++) {
+                    const cf cv = c[k], hv = h[k * hs];
+                    mu = __fmaf_rn(cv.x, hv.x, mu);
+                    mu = __fmaf_rn(-cv.y, hv.y, mu);
+                }
+                const float ni = __fdiv_rn(mu, __fsub_rn(1.0f, mu));
+                float* f = reinterpret_cast<float*>(sh + j * ts + m.l + L * L) + L;
+                f[l] = __fdiv_rn(1.0f, mu);
+                f[L + l] = ni;
+                if (MODE == kCoef && sc0 + j < cl.nSC) cl.nInv[(sc0 + j) * L + l] = ni;
             }
-            const float ni = __fdiv_rn(mu, __fsub_rn(1.0f, mu));
-            sMuInv[tid] = __fdiv_rn(1.0f, mu);
-            sNoise[tid] = ni;
-            if (MODE == kCoef && out) cl.nInv[sc * L + tid] = ni;
         }
-        team_sync<TEAM>();
-        for (int l = 0; l < L; l++) {
+        __syncthreads();
+        if constexpr (MODE == kChain) {                // H is spent: Y takes its place
+            stage_rows<TEAM>(sY, cs, cl.Y + sc * S * A, S, A, cl.vecY, tid);
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        }
+        const float* sMuInv = sInv + L;
+#pragma unroll
+        for (int l = 0; l < LT; l++) {
+            if (!EX && l >= L) break;
             const float im = sMuInv[l];
             for (int k = tid; k < A; k += TEAM) {
                 const cf v = sC[l * cs + k];
@@ -368,15 +414,15 @@ __global__ void __launch_bounds__(128) plain_kernel(const __grid_constant__ Plai
             }
         }
         if constexpr (MODE == kCoef) return;
+        noise = sMuInv[L + min(tid / LPL, L - 1)];
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
 
     // ---- Y_eq (and LLRs): lane (layer l, symbols st, st + LPL, ...) ----
     if constexpr (MODE != kCoef) {
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         team_sync<TEAM>();
         const int l = tid / LPL, st = tid % LPL;
         if (l >= L) return;
-        if constexpr (MODE == kChain) noise = sNoise[l];
         switch ((S + LPL - 1) / LPL) {
             case 1: apply_symbols<MODE, 1, LPL>(cl, sC, sY, cs, noise, sc, l, st, out); break;
             case 2: apply_symbols<MODE, 2, LPL>(cl, sC, sY, cs, noise, sc, l, st, out); break;
@@ -630,13 +676,17 @@ static int layers_tile(int L) { return L <= 2 ? 2 : L <= 4 ? 4 : L <= 8 ? 8 : 16
 template <int MODE, int LT, bool EX>
 static int launch_plain_t(PlainParams& p, cudaStream_t st) {
     constexpr int TEAM = plain_team(LT);
-    int teamBytes = 0;
+    int values = 0;
     for (int i = 0; i < p.nCells; i++)
-        teamBytes = std::max(teamBytes, plain_team_bytes(MODE, p.cell[i].A, p.cell[i].L, p.cell[i].S));
-    // 128 threads a block, fewer (whole warps) where their rows do not fit:
-    // the largest team's need (256 antennas, 16 layers, 16 symbols) is 103 KB
+        values = std::max(values, plain_smem(MODE, p.cell[i].A, p.cell[i].L, p.cell[i].S).total);
+    // the subcarriers of a block that one warp reads together start LT values
+    // apart in the banks
+    if (LT < 16) values += (LT - values % 16 + 16) % 16;
+    const int teamBytes = values * (int)sizeof(cf);
+    // fewer teams (whole warps) where their rows do not fit: the largest team's
+    // need (256 antennas, 16 layers, 16 symbols) is 72 KB
     constexpr int WARP_TEAMS = TEAM >= 32 ? 1 : 32 / TEAM;
-    int teams = 128 / TEAM;
+    int teams = kPlainThreads / TEAM;
     while (teams > WARP_TEAMS && teams * teamBytes > kMaxSmemPerCta) teams -= WARP_TEAMS;
     if (teams * teamBytes > kMaxSmemPerCta) return AERIAL_ERR_UNSUPPORTED;
     const int s = allow_max_smem<plain_kernel<MODE, LT, EX>>();
@@ -646,7 +696,7 @@ static int launch_plain_t(PlainParams& p, cudaStream_t st) {
         p.cell[i].block0 = blocks;
         blocks += (unsigned)((p.cell[i].nSC + teams - 1) / teams);
     }
-    p.teamBytes = teamBytes;
+    p.teamValues = values;
     plain_kernel<MODE, LT, EX><<<blocks, teams * TEAM, (size_t)teams * teamBytes, st>>>(p);
     return launch_status();
 }
