@@ -358,44 +358,92 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) chest_umma_kernel(const __gri
     const long M = (long)nBlocks * nAnt;
     const long nMT = (M + kUmmaM - 1) / kUmmaM;
 
+    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + 2), tfull0 = smem_u32(bars + 4),
+                   tempty0 = smem_u32(bars + 6);
+    // A tile of M tile mt into stage st (one thread).
+    auto load_tile = [&](long mt, int st) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(full0 + 8 * st), "r"(aStage)
+                     : "memory");
+        for (int q = 0; q < nSrs; q++)
+#pragma unroll
+            for (int kb = 0; kb < KB; kb++)
+                asm volatile(
+                    "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+                    "[%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(
+                        smem_u32(sA + st * aStage + (uint32_t)(q * KB + kb) * kUmmaAtomBytes)),
+                    "l"(reinterpret_cast<uint64_t>(&tmA)), "r"(kb * kUmmaKB), "r"((int)(mt * kUmmaM)), "r"(q),
+                    "r"(full0 + 8 * st)
+                    : "memory");
+    };
     if (threadIdx.x == 0) {
         for (int b = 0; b < 8; b++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bars + b)),
                          "r"(b >= 6 ? kUmmaEpiWarps : 1));   // tempty: one arrival per epilogue warp
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // the copies see the barriers
+        // the first two tiles arrive while the taps are built (the barriers
+        // are this thread's own so far)
+        for (int st = 0; st < 2; st++)
+            if (blockIdx.x + (long)st * gridDim.x < nMT) load_tile(blockIdx.x + (long)st * gridDim.x, st);
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tslot)),
                      "r"(kTCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
-    // B's K columns past 2 nPilot inside the last atom must read as zero
-    for (int e = threadIdx.x; e < 2 * KB * kBAtom / 16; e += blockDim.x)
-        reinterpret_cast<uint4*>(sB)[e] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
     // B tile: rows r = 2 j + (re/im output) for complex output n = NTL/2 nt + j,
-    // K columns 2 kc + (re/im input); (Re T, -Im T) / (Im T, Re T) pairs.
-    for (int e = threadIdx.x; e < (NTL / 2) * nPilot; e += blockDim.x) {
-        const int j = e / nPilot, kc = e - j * nPilot;
-        const int n = (NTL / 2) * nt + j;
-        float2 t = make_float2(0.f, 0.f);
-        if (n < N) {
-            const float2 w = __half22float2(Wf[(n / P) * nPilot + kc]);
-            const float2 f = __half22float2(occ[(n % P) * F + (kc % F)]);
-            t = make_float2(w.x * f.x - w.y * f.y, w.x * f.y + w.y * f.x);
-            if (nSrs > 1) t = make_float2(t.x * (1.f / nSrs), t.y * (1.f / nSrs));   // a power of two: exact
+    // K columns 2 kc + (re/im input); (Re T, -Im T) / (Im T, Re T) pairs, zeros
+    // past nPilot to the end of the last atom (whose columns meet the A box's
+    // zero fill) and past N.  A warp builds an output's rows, lane = tap: the
+    // loads of a row of Wf and the stores of a row of B are contiguous, and a
+    // lane's cover code indices are the same for every output.  One tap per
+    // thread with divisions for its indices, after a pass that zeroed B, and the
+    // first copies only then: 13.5 us for a launch of one tile per CTA with 96
+    // pilots, 8.3 us as here (2,720 blocks 116 -> 111 us, the SRS filter's
+    // 2,960 blocks 23.5 -> 21.9 us and 10,560 blocks 62.2 -> 61.8 us).
+    {
+        constexpr int NW = kUmmaThreads / 32, JU = 4;         // outputs whose loads go out together
+        int fi[KB];
+#pragma unroll
+        for (int kb = 0; kb < KB; kb++) fi[kb] = (kb * 32 + lane) % F;
+        const float scale = 1.f / nSrs;                       // a power of two: exact
+#pragma unroll 1
+        for (int j0 = warp; j0 < NTL / 2; j0 += NW * JU) {
+            __half2 w[JU][KB], f[JU][KB];
+#pragma unroll
+            for (int u = 0; u < JU; u++) {
+                const int j = j0 + u * NW, n = (NTL / 2) * nt + j;
+                const int o = n / P, port = n - o * P;
+#pragma unroll
+                for (int kb = 0; kb < KB; kb++) {
+                    const int kc = kb * 32 + lane;
+                    const bool in = j < NTL / 2 && n < N && kc < nPilot;
+                    w[u][kb] = in ? Wf[o * nPilot + kc] : __half2{};
+                    f[u][kb] = in ? occ[port * F + fi[kb]] : __half2{};
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < JU; u++) {
+                const int j = j0 + u * NW;
+                if (j >= NTL / 2) break;
+#pragma unroll
+                for (int kb = 0; kb < KB; kb++) {
+                    const float2 a = __half22float2(w[u][kb]), c = __half22float2(f[u][kb]);
+                    float2 t = make_float2(a.x * c.x - a.y * c.y, a.x * c.y + a.y * c.x);
+                    if (nSrs > 1) t = make_float2(t.x * scale, t.y * scale);
+                    uint32_t hi0, lo0, hi1, lo1;
+                    split_h2(t.x, -t.y, hi0, lo0);           // row 2j: Re out
+                    split_h2(t.y, t.x, hi1, lo1);            // row 2j+1: Im out
+                    uint8_t* bh = sB + kb * kBAtom;
+                    uint8_t* bl = sB + (KB + kb) * kBAtom;
+                    *reinterpret_cast<uint32_t*>(bh + sw128_off(2 * j, 2 * lane)) = hi0;
+                    *reinterpret_cast<uint32_t*>(bl + sw128_off(2 * j, 2 * lane)) = lo0;
+                    *reinterpret_cast<uint32_t*>(bh + sw128_off(2 * j + 1, 2 * lane)) = hi1;
+                    *reinterpret_cast<uint32_t*>(bl + sw128_off(2 * j + 1, 2 * lane)) = lo1;
+                }
+            }
         }
-        uint32_t hi0, lo0, hi1, lo1;
-        split_h2(t.x, -t.y, hi0, lo0);           // row 2j: Re out
-        split_h2(t.y, t.x, hi1, lo1);            // row 2j+1: Im out
-        const int k = 2 * kc, kb = k >> 6, kin = k & 63;
-        uint8_t* bh = sB + kb * kBAtom;
-        uint8_t* bl = sB + (KB + kb) * kBAtom;
-        *reinterpret_cast<uint32_t*>(bh + sw128_off(2 * j, kin)) = hi0;
-        *reinterpret_cast<uint32_t*>(bl + sw128_off(2 * j, kin)) = lo0;
-        *reinterpret_cast<uint32_t*>(bh + sw128_off(2 * j + 1, kin)) = hi1;
-        *reinterpret_cast<uint32_t*>(bl + sw128_off(2 * j + 1, kin)) = lo1;
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -403,27 +451,14 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) chest_umma_kernel(const __gri
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tbase = *tslot;
 
-    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + 2), tfull0 = smem_u32(bars + 4),
-                   tempty0 = smem_u32(bars + 6);
     if (warp == 0) {
         if (lane == 0) {
-            long i = 0;
-            for (long mt = blockIdx.x; mt < nMT && !*abort; mt += gridDim.x, i++) {
+            // tiles 0 and 1 are under way since the start
+            long i = min(2L, (nMT - blockIdx.x + gridDim.x - 1) / gridDim.x);
+            for (long mt = blockIdx.x + i * gridDim.x; mt < nMT && !*abort; mt += gridDim.x, i++) {
                 const int s = (int)(i & 1);
                 if (!mbar_wait(empty0 + 8 * s, (uint32_t)(((i >> 1) & 1) ^ 1), abort)) break;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(full0 + 8 * s),
-                             "r"(aStage)
-                             : "memory");
-                for (int q = 0; q < nSrs; q++)
-#pragma unroll
-                    for (int kb = 0; kb < KB; kb++)
-                        asm volatile(
-                            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                            "[%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(
-                                smem_u32(sA + s * aStage + (uint32_t)(q * KB + kb) * kUmmaAtomBytes)),
-                            "l"(reinterpret_cast<uint64_t>(&tmA)), "r"(kb * kUmmaKB), "r"((int)(mt * kUmmaM)), "r"(q),
-                            "r"(full0 + 8 * s)
-                            : "memory");
+                load_tile(mt, s);
             }
             // leave no copy in flight: the last two stages' loads have landed
             for (long d = (i > 2 ? i - 2 : 0); d < i; d++) mbar_wait(full0 + 8 * (d & 1), (uint32_t)((d >> 1) & 1), abort);
