@@ -169,12 +169,34 @@ __device__ __forceinline__ float2 sub2(float re, float im, float2 h) {
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk2(re, im)), "l"(pk2(h.x, h.y)));
     return upk2(d);
 }
-// bf16 hi/lo split of a complex pair: x = hi + lo to ~16 mantissa bits.
+// h - x of a packed bfloat16 pair, straight from its halves: widening them
+// takes two instructions per pair on the integer pipe, which a split for 16
+// layers or in a mixed launch keeps half busy as it is (half precision widens
+// on the FP32 pipe).  BF16X3 operands: 12-slot precision-stress launch 299 us
+// with that, 285 us as here, 24 uneven cells 56 and 53 us.  Uniform launches
+// of up to 8 layers wait for memory, not for that pipe, and two subtractions
+// in place of one packed one cost them 2 % (16 slots of 132 PRB x 64 antennas x
+// 8 layers 66 and 68 us), so they keep the packed form (split2).
+__device__ __forceinline__ float2 sub_bf16(uint32_t h, float re, float im) {
+    float2 d;
+    asm("{\n .reg .b16 a, b;\n mov.b32 {a, b}, %2;\n sub.rn.f32.bf16 %0, a, %3;\n sub.rn.f32.bf16 %1, b, %4;\n}\n"
+        : "=f"(d.x), "=f"(d.y)
+        : "r"(h), "f"(re), "f"(im));
+    return d;
+}
+// bf16 hi/lo split of a complex pair: x = hi + lo to ~16 mantissa bits.  The
+// same bits either way.
+template <bool HALVES>
 __device__ __forceinline__ void split_bf16(float re, float im, uint32_t& hi, uint32_t& lo) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(re, im);
-    const float2 r = sub2(re, im, __bfloat1622float2(h));
-    __nv_bfloat162 l = __floats2bfloat162_rn(r.x, r.y);
+    __nv_bfloat162 h = __floats2bfloat162_rn(re, im), l;
     hi = *reinterpret_cast<uint32_t*>(&h);
+    if constexpr (HALVES) {
+        const float2 r = sub_bf16(hi, re, im);           // -lo, before its rounding
+        l = __floats2bfloat162_rn(-r.x, -r.y);
+    } else {
+        const float2 r = sub2(re, im, __bfloat1622float2(h));
+        l = __floats2bfloat162_rn(r.x, r.y);
+    }
     lo = *reinterpret_cast<uint32_t*>(&l);
 }
 // fp16 hi/lo split: x = hi + lo to ~22 significant bits, for operands the
@@ -186,12 +208,12 @@ __device__ __forceinline__ void split_fp16(float re, float im, uint32_t& hi, uin
     hi = *reinterpret_cast<uint32_t*>(&h);
     lo = *reinterpret_cast<uint32_t*>(&l);
 }
-template <int P>
+template <int P, bool HALVES>
 __device__ __forceinline__ void split2(float re, float im, uint32_t& hi, uint32_t& lo) {
     if constexpr (P == AERIAL_PREC_FP16X3)
         split_fp16(re, im, hi, lo);
     else
-        split_bf16(re, im, hi, lo);
+        split_bf16<HALVES>(re, im, hi, lo);
 }
 
 template <int P>
@@ -348,6 +370,7 @@ __device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, const
                                           float (*gacc)[4], float (*zacc)[2][4], bool z2, int g, int c,
                                           unsigned long long ss = 0) {
     constexpr int NMT = LT > 8 ? 2 : 1;
+    constexpr bool HALVES = LT == 16 || NZ == 0;         // 16 layers, or a mixed launch
 #pragma unroll
     for (int kk = 0; kk < 2; kk++) {
         const int a0 = 8 * kk + 2 * c;
@@ -375,15 +398,15 @@ __device__ __forceinline__ void mma_stage(uint32_t st, int hrs, int nRows, const
             uint32_t ah[NMT][2], al[NMT][2];
 #pragma unroll
             for (int mt = 0; mt < NMT; mt++) {
-                split2<P>(hv[mt].x, hv[mt].y, ah[mt][0], al[mt][0]);
-                split2<P>(hv[mt].z, hv[mt].w, ah[mt][1], al[mt][1]);
+                split2<P, HALVES>(hv[mt].x, hv[mt].y, ah[mt][0], al[mt][0]);
+                split2<P, HALVES>(hv[mt].z, hv[mt].w, ah[mt][1], al[mt][1]);
             }
             uint32_t yh[2][2], yl[2][2];
 #pragma unroll
             for (int nt = 0; nt < 2; nt++) {
                 if (NZ == 1 && nt == 1) break;
-                split2<P>(yv[nt].x, yv[nt].y, yh[nt][0], yl[nt][0]);
-                split2<P>(yv[nt].z, yv[nt].w, yh[nt][1], yl[nt][1]);
+                split2<P, HALVES>(yv[nt].x, yv[nt].y, yh[nt][0], yl[nt][0]);
+                split2<P, HALVES>(yv[nt].z, yv[nt].w, yh[nt][1], yl[nt][1]);
             }
 #pragma unroll
             for (int mt = 0; mt < NMT; mt++) {
