@@ -48,6 +48,7 @@ constexpr int kTcSteps = 4;
 template <int NMT, int NNT, bool VEC>
 __global__ void __launch_bounds__(256) coef_apply_tc_kernel(const float2* __restrict__ C, const float2* __restrict__ Y,
                                                              float2* __restrict__ O, int nSC, int nSym, int L, int A) {
+    wait_previous();
     const int lane = threadIdx.x & 31;
     const int g = lane >> 2, c = lane & 3;
     const long w0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -104,12 +105,12 @@ __global__ void __launch_bounds__(256) coef_apply_tc_kernel(const float2* __rest
 }
 
 template <int NMT, int NNT>
-static void launch_tc(const float2* C, const float2* Y, float2* O, int nSC, int nSym, int L, int A, bool vec,
+static int launch_tc(const float2* C, const float2* Y, float2* O, int nSC, int nSym, int L, int A, bool vec,
                       cudaStream_t st) {
     // a warp per subcarrier, at most the two 256-thread blocks an SM holds at a time, twice over
     const unsigned blocks = (unsigned)std::min(((long)nSC + 7) / 8, (long)sm_count() * 8);
-    if (vec) coef_apply_tc_kernel<NMT, NNT, true><<<blocks, 256, 0, st>>>(C, Y, O, nSC, nSym, L, A);
-    else coef_apply_tc_kernel<NMT, NNT, false><<<blocks, 256, 0, st>>>(C, Y, O, nSC, nSym, L, A);
+    return launch_after(vec ? coef_apply_tc_kernel<NMT, NNT, true> : coef_apply_tc_kernel<NMT, NNT, false>, blocks, 256, 0,
+                        st, C, Y, O, nSC, nSym, L, A);
 }
 
 }  // namespace aeq
@@ -124,6 +125,5 @@ extern "C" int aerial_coef_apply_tc(const aerial_cf32* C, const aerial_cf32* Y_r
     const bool vec = (nAnt % 2) == 0 && ((uintptr_t)C & 15) == 0 && ((uintptr_t)Y_rx & 15) == 0;
     auto run = nLayers > 8 ? (nSym > 8 ? launch_tc<2, 2> : launch_tc<2, 1>)
                            : (nSym > 8 ? launch_tc<1, 2> : launch_tc<1, 1>);
-    run((const float2*)C, (const float2*)Y_rx, (float2*)Y_eq, nSC, nSym, nLayers, nAnt, vec, to_stream(stream));
-    return launch_status();
+    return run((const float2*)C, (const float2*)Y_rx, (float2*)Y_eq, nSC, nSym, nLayers, nAnt, vec, to_stream(stream));
 }

@@ -929,6 +929,7 @@ __device__ __forceinline__ int group_valid(const FusedCell& cl, long grp) {
 // SC: the launch has cells whose FP16 operands are scaled (mma_stage).
 template <int P, int LTF, bool SC = false>
 __global__ void __launch_bounds__(256, 2) fused_eq_kernel(const __grid_constant__ FusedParams p) {
+    wait_previous();
     extern __shared__ float4 smem_raw[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -1191,6 +1192,7 @@ __device__ __forceinline__ void run_group(const FusedParams& p, MixedWarp& w, in
 
 template <int P, bool SC = false>
 __global__ void __launch_bounds__(256, 2) fused_eq_kernel_m(const __grid_constant__ FusedParams p) {
+    wait_previous();
     extern __shared__ float4 smem_raw[];
     const int wib = threadIdx.x >> 5;
     const int warpsPerCta = blockDim.x >> 5;
@@ -1282,6 +1284,7 @@ __device__ __forceinline__ void stage_chunk(uint32_t st, uint32_t hLaneS, uint32
 // same box, bit-identical.
 template <int P, int LTF, int NCH, bool SC = false>
 __global__ void __launch_bounds__(256, LTF == 16 ? 1 : 2) fused_eq_kernel_a(const __grid_constant__ FusedParams p) {
+    wait_previous();
     constexpr int NST = stages_of_a(LTF, NCH);
     constexpr int A = CHUNK * NCH;
     constexpr int HRS = hrs_of(LTF);
@@ -1506,6 +1509,7 @@ __device__ __forceinline__ void mma_stage_h(uint32_t st, uint32_t hb, const uint
 
 template <int LTF, int NCH>
 __global__ void __launch_bounds__(256, 2) fused_eq_kernel_h(const __grid_constant__ FusedParams p) {
+    wait_previous();
     constexpr int NST = stages_of_a(LTF, NCH);
     constexpr int A = CHUNK * NCH;
     constexpr int HRS = hrs16_of(LTF);
@@ -1675,6 +1679,7 @@ __host__ __device__ constexpr uint32_t h_lane_stage(int LT, int lane) {
 }
 
 __global__ void __launch_bounds__(256, 2) fused_eq_kernel_hg(const __grid_constant__ FusedParams p) {
+    wait_previous();
     constexpr int NST = 2;
     extern __shared__ float4 smem_raw[];
     const int lane = threadIdx.x & 31;
@@ -2341,8 +2346,8 @@ int launch_fused(FusedParams& p, int warpBytes, int prec, LaunchShape sh, cudaSt
     WalkTable* t = walk_applies(p, pl) ? walk_table_locked(lk) : nullptr;
     p.walkSlot = t ? walk_slot_for_stream(t, st) : -1;
     void* args[] = {&p};
-    const cudaError_t e = cudaLaunchKernel(pl.func, pl.grid, pl.block, args, (size_t)pl.smem, st);
-    if (e != cudaSuccess) return rt_status(e);
+    s = launch_after(pl.func, pl.grid, pl.block, (size_t)pl.smem, st, args);
+    if (s) return s;
     return p.walkSlot >= 0 ? walk_record(t, p.walkSlot, st) : AERIAL_OK;
 }
 

@@ -296,6 +296,7 @@ __global__ void __launch_bounds__(kPlainThreads) plain_kernel(const __grid_const
     constexpr int TEAM = plain_team(LT);
     constexpr int LPL = TEAM / LT;                     // lanes per layer of the apply phase
     extern __shared__ float4 plain_shared[];
+    wait_previous();
     const int team = threadIdx.x / TEAM, tid = threadIdx.x % TEAM, teams = blockDim.x / TEAM;
     int ci = 0;
     while (ci + 1 < p.nCells && blockIdx.x >= p.cell[ci + 1].block0) ci++;
@@ -465,6 +466,7 @@ template <int LT, bool EX>
 __global__ void __launch_bounds__(kGramThreads) gram_kernel(const GramParams p) {
     constexpr int RT = gram_rt(LT), CT = gram_ct(LT), TEAM = gram_team(LT), PER = 32 / TEAM;
     extern __shared__ float4 gram_smem[];
+    wait_previous();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int A = p.A, L = EX ? LT : p.L, hs = EX ? LT + 2 : plain_hs(L);
     const int ts = (A + 1) * hs;                       // values per subcarrier
@@ -607,6 +609,7 @@ __global__ void __launch_bounds__(kLlrThreads) llr_f16_kernel(const __half2* __r
                                                                const float* __restrict__ ni,
                                                                __half* __restrict__ out, int count, bool wide,
                                                                PamLut lut) {
+    wait_previous();
     __half2 v[kLlrPerThread];
     float nv[kLlrPerThread];
     const long base = (long)blockIdx.x * kLlrThreads * kLlrPerThread;
@@ -638,6 +641,7 @@ __global__ void __launch_bounds__(kLlrThreads) llr_f32_kernel(const cf* __restri
                                                                const float* __restrict__ ni,
                                                                float* __restrict__ out, int count, int symsPerNoise,
                                                                unsigned rcp, bool wide, PamLut lut) {
+    wait_previous();
     cf v[kLlrPerThread];
     float nv[kLlrPerThread];
     const long base = (long)blockIdx.x * kLlrThreads * kLlrPerThread;
@@ -697,8 +701,7 @@ static int launch_plain_t(PlainParams& p, cudaStream_t st) {
         blocks += (unsigned)((p.cell[i].nSC + teams - 1) / teams);
     }
     p.teamValues = values;
-    plain_kernel<MODE, LT, EX><<<blocks, teams * TEAM, (size_t)teams * teamBytes, st>>>(p);
-    return launch_status();
+    return launch_after(plain_kernel<MODE, LT, EX>, blocks, teams * TEAM, (size_t)teams * teamBytes, st, p);
 }
 
 template <int MODE, int LT>
@@ -741,8 +744,7 @@ static int launch_gram_t(const GramParams& p, cudaStream_t st) {
     while (warps > 1 && warps * warpBytes > (size_t)kMaxSmemPerCta) warps--;   // one warp needs 131 KB at most
     const long perBlock = (long)warps * (32 / gram_team(LT));
     const unsigned blocks = (unsigned)((p.nSC + perBlock - 1) / perBlock);
-    gram_kernel<LT, EX><<<blocks, warps * 32, warps * warpBytes, st>>>(p);
-    return launch_status();
+    return launch_after(gram_kernel<LT, EX>, blocks, warps * 32, warps * warpBytes, st, p);
 }
 
 static int launch_gram(const cf* H, float sigma2, cf* G, int nSC, int A, int L, cudaStream_t st) {
@@ -788,12 +790,11 @@ static int launch_llr_f32(const cf* in, const float* ni, float* out, int N, int 
     const unsigned rcp = spn > 1 ? (unsigned)(0x100000000ull / (unsigned)spn) + 1u : 0u;
     const bool w = llr_wide(out, 2 * n);
     switch (n) {
-        case 1: llr_f32_kernel<1><<<g, kLlrThreads, 0, st>>>(in, ni, out, N, spn, rcp, w, lut); break;
-        case 2: llr_f32_kernel<2><<<g, kLlrThreads, 0, st>>>(in, ni, out, N, spn, rcp, w, lut); break;
-        case 3: llr_f32_kernel<3><<<g, kLlrThreads, 0, st>>>(in, ni, out, N, spn, rcp, w, lut); break;
-        default: llr_f32_kernel<4><<<g, kLlrThreads, 0, st>>>(in, ni, out, N, spn, rcp, w, lut); break;
+        case 1: return launch_after(llr_f32_kernel<1>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
+        case 2: return launch_after(llr_f32_kernel<2>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
+        case 3: return launch_after(llr_f32_kernel<3>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
+        default: return launch_after(llr_f32_kernel<4>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
     }
-    return launch_status();
 }
 
 }  // namespace aeq
@@ -878,12 +879,11 @@ extern "C" int aerial_llr(const aerial_ch2* softEst, const float* noiseInv, uint
     __half* out = (__half*)llrOut;
     const bool w = llr_wide(out, nPamBits);
     switch (nPamBits) {
-        case 1: llr_f16_kernel<1><<<g, kLlrThreads, 0, st>>>(in, noiseInv, out, N, w, lut); break;
-        case 2: llr_f16_kernel<2><<<g, kLlrThreads, 0, st>>>(in, noiseInv, out, N, w, lut); break;
-        case 3: llr_f16_kernel<3><<<g, kLlrThreads, 0, st>>>(in, noiseInv, out, N, w, lut); break;
-        default: llr_f16_kernel<4><<<g, kLlrThreads, 0, st>>>(in, noiseInv, out, N, w, lut); break;
+        case 1: return launch_after(llr_f16_kernel<1>, g, kLlrThreads, 0, st, in, noiseInv, out, N, w, lut);
+        case 2: return launch_after(llr_f16_kernel<2>, g, kLlrThreads, 0, st, in, noiseInv, out, N, w, lut);
+        case 3: return launch_after(llr_f16_kernel<3>, g, kLlrThreads, 0, st, in, noiseInv, out, N, w, lut);
+        default: return launch_after(llr_f16_kernel<4>, g, kLlrThreads, 0, st, in, noiseInv, out, N, w, lut);
     }
-    return launch_status();
 }
 
 extern "C" int aerial_llr_f32(const aerial_cf32* softEst, const float* noiseInv, float* llrOut, int N, int nPamBits,

@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(kSrsWarps * 32, 2) srs_filter_tc_kernel(const 
                                                                           const __half2* __restrict__ focc,
                                                                           void* __restrict__ out, int nAnt,
                                                                           int nBlocks, int K, int Ko, int P, int F, int NQ) {
+    wait_previous();
     extern __shared__ uint4 bfrag[];            // [group][kstep][tile][lane]: {b0 hi, b1 hi, b0 lo, b1 lo}
     const int N = Ko * P;                        // complex outputs per antenna
     const int nGroups = (N + 15) / 16;
@@ -340,6 +341,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) chest_umma_kernel(const __gri
                                                                       void* __restrict__ out, int nAnt, int nBlocks,
                                                                       int nPilot, int nOut, int P, int F, int nSrs) {
     extern __shared__ __align__(1024) uint8_t usm_raw[];
+    wait_previous();
     // 128-byte swizzle atoms must start on 1024-byte boundaries of the shared window
     uint8_t* usm = usm_raw + ((1024u - (smem_u32(usm_raw) & 1023u)) & 1023u);
     // layout: A stages [2][nSrs x KB atoms of 128 rows] | B [hi, lo][KB atoms of NTL rows] | barriers | TMEM slot
@@ -668,9 +670,8 @@ static int launch_chest_umma(void* out, const aerial_ch2* Yp, const aerial_ch2* 
     long gx = std::max(1L, (long)sm_count() / nNT);
     gx = std::min(gx, nMT);
     dim3 grid((unsigned)gx, (unsigned)nNT);
-    chest_umma_kernel<KB, NTL, OUTL><<<grid, kUmmaThreads, smem, st>>>(tm, (const __half2*)Wf, (const __half2*)OCC, out,
-                                                                   nAnt, nBlocks, nPilot, nOut, P, F, nSrs);
-    return launch_status();
+    return launch_after(chest_umma_kernel<KB, NTL, OUTL>, grid, kUmmaThreads, smem, st, tm, (const __half2*)Wf,
+                        (const __half2*)OCC, out, nAnt, nBlocks, nPilot, nOut, P, F, nSrs);
 }
 
 // The filter on tcgen05 when the shape allows it; AERIAL_ERR_UNSUPPORTED
@@ -715,9 +716,8 @@ static int launch_srs_tc(void* out, const aerial_ch2* SRS, const aerial_ch2* W, 
     long gx = std::max(1L, (long)sm_count() * std::max(1, perSm) / slices);
     gx = std::min(gx, ctasForItems);
     dim3 grid((unsigned)gx, (unsigned)slices);
-    kern<<<grid, kSrsWarps * 32, smem, st>>>((const __half2*)SRS, (const __half2*)W, (const __half2*)FOCC, out,
-                                             nAnt, nBlocks, K, Ko, P, F, NQ);
-    return launch_status();
+    return launch_after(kern, grid, kSrsWarps * 32, smem, st, (const __half2*)SRS, (const __half2*)W, (const __half2*)FOCC,
+                        out, nAnt, nBlocks, K, Ko, P, F, NQ);
 }
 
 // H_est layout (the SRS filter): up to 48 taps.
