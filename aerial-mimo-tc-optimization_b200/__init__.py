@@ -347,7 +347,7 @@ def pusch_eq_plain_workspace(cells) -> int:
 
 
 def pusch_eq_plain(cells, workspace, stream=None):
-    """The plain FP32 chain (gram, mmse_coef, coef_apply, llr_f32 per cell)."""
+    """The plain FP32 chain (gram, mmse_coef, coef_apply, llr_f32 of each cell, in one kernel)."""
     arr, n = _cells_array(cells)
     _check(lib().aerial_pusch_eq_plain(arr, n, _ptr(workspace), workspace.numel() * workspace.element_size(),
                                        _stream(stream)), "pusch_eq_plain")
@@ -355,8 +355,8 @@ def pusch_eq_plain(cells, workspace, stream=None):
 
 def pusch_eq_plain_static(cells, stream=None):
     """The plain FP32 chain without a workspace argument, for callers that cannot
-    allocate device memory: intermediates live in the library's static 16 MiB
-    device array (shared by all calls; calls overlapping on the GPU race)."""
+    allocate device memory; cells with more than 16 MiB of intermediates are
+    refused."""
     arr, n = _cells_array(cells)
     _check(lib().aerial_pusch_eq_plain_static(arr, n, _stream(stream)), "pusch_eq_plain_static")
 

@@ -13,7 +13,9 @@
  *   - Buffers are DEVICE pointers owned by the caller unless stated
  *     otherwise; nothing is allocated, freed or synchronised by a call.
  *   - `stream` is a cudaStream_t passed as void* (NULL = legacy default
- *     stream).  Work is enqueued asynchronously on it.
+ *     stream).  Work is enqueued asynchronously on it, behind everything
+ *     enqueued before (kernels are launched with programmatic stream
+ *     serialization and wait for the stream on the device).
  *   - Return value: AERIAL_OK (0), an AERIAL_ERR_* code for bad arguments,
  *     or a cudaError_t value (1..999) from the launch.  Nothing calls
  *     exit(); the reference's CUDA_CHECK -> exit(1) becomes a status.
@@ -308,10 +310,12 @@ int aerial_pusch_eq_host_workspace(const aerial_cell_desc* cells, int nCells, in
 int aerial_pusch_eq_host(const aerial_cell_desc* cells, int nCells, const aerial_tuning* tuning,
                          int cellsPerBatch, void* workspace, size_t workspaceBytes, void* stream);
 
-/* The plain FP32 chain for the same cells: aerial_gram, aerial_mmse_coef,
- * aerial_coef_apply and aerial_llr_f32 per cell, intermediates in the
- * caller's workspace (size from aerial_pusch_eq_plain_workspace).  This is
- * the reference's stage-by-stage scalar method on the GPU. */
+/* The plain FP32 chain for the same cells: the results of aerial_gram,
+ * aerial_mmse_coef, aerial_coef_apply and aerial_llr_f32 per cell, bit for bit,
+ * which is the reference's stage-by-stage scalar method on the GPU.  One kernel
+ * runs all stages with the intermediates on chip; the workspace (size from
+ * aerial_pusch_eq_plain_workspace) is checked and left as it is.  Every cell
+ * is checked before anything is launched. */
 size_t aerial_pusch_eq_plain_workspace(const aerial_cell_desc* cells, int nCells);
 int aerial_pusch_eq_plain(const aerial_cell_desc* cells, int nCells, void* workspace,
                           size_t workspaceBytes, void* stream);
@@ -319,19 +323,14 @@ int aerial_pusch_eq_plain(const aerial_cell_desc* cells, int nCells, void* works
 /* The plain chain for callers that cannot allocate device memory -- a
  * real-time slot loop where cudaMalloc may block or synchronize the device,
  * or a plugin whose host framework owns all device memory.  No counterpart in
- * the reference.  Same cells and results as aerial_pusch_eq_plain, but the
- * intermediates live in one static device array of
- * AERIAL_STATIC_SCRATCH_BYTES (16 MiB) inside this library, held on every GPU
- * that loads it until exit; a batch whose largest cell needs more (see
- * aerial_pusch_eq_plain_workspace; e.g. a 273-PRB, 128-antenna, 16-layer
- * cell) is rejected with AERIAL_ERR_SCRATCH_LIMIT before anything runs.
- * Malformed cells return AERIAL_ERR_INVALID_ARG (or AERIAL_ERR_UNSUPPORTED
- * for a complex-half cell) before the size check.  The first call in each
- * CUDA context looks up the array's device address: once per device, and
- * again after a cudaDeviceReset or in a second context on the same device,
- * each of which holds its own copy of the array (make that call before any
- * stream capture).  Calls share the array, so calls that overlap on the GPU
- * race; nothing is allocated or freed. */
+ * the reference.  Same cells and results as aerial_pusch_eq_plain, with no
+ * device memory but the cells' own; calls may overlap on the GPU.  A batch
+ * whose largest cell has intermediates of more than
+ * AERIAL_STATIC_SCRATCH_BYTES (16 MiB; see aerial_pusch_eq_plain_workspace;
+ * e.g. a 273-PRB, 128-antenna, 16-layer cell) is rejected with
+ * AERIAL_ERR_SCRATCH_LIMIT before anything runs.  Malformed cells return
+ * AERIAL_ERR_INVALID_ARG (or AERIAL_ERR_UNSUPPORTED for a complex-half cell)
+ * before the size check. */
 #define AERIAL_STATIC_SCRATCH_BYTES (16u << 20)
 int aerial_pusch_eq_plain_static(const aerial_cell_desc* cells, int nCells, void* stream);
 
