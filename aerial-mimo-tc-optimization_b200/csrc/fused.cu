@@ -1250,6 +1250,14 @@ __global__ void __launch_bounds__(256, 2) fused_eq_kernel_m(const __grid_constan
 __host__ __device__ constexpr int stages_of_a(int ltf, int nch) {
     return stages_of(ltf) < nch + 1 ? stages_of(ltf) : nch + 1;
 }
+// Complex-half stages are half the size: four of them (two for 16 layers) still
+// leave 16 resident warps, and the copies further ahead.  64 slots of 132 PRB x
+// 64 antennas x 8 layers 139 us with three, 133 us with four; 16 of 106 x 128 x
+// 8 55 and 53 us; 16 of 273 x 64 x 4 60 and 57.5 us.
+__host__ __device__ constexpr int stages_of_h(int ltf, int nch) {
+    const int n = ltf == 16 ? 2 : 4;
+    return n < nch + 1 ? n : nch + 1;
+}
 
 // One subcarrier's operands as the producing lane sees them: its first
 // channel piece, its first received piece, its count of received rows.
@@ -1510,7 +1518,7 @@ __device__ __forceinline__ void mma_stage_h(uint32_t st, uint32_t hb, const uint
 template <int LTF, int NCH>
 __global__ void __launch_bounds__(256, 2) fused_eq_kernel_h(const __grid_constant__ FusedParams p) {
     wait_previous();
-    constexpr int NST = stages_of_a(LTF, NCH);
+    constexpr int NST = stages_of_h(LTF, NCH);
     constexpr int A = CHUNK * NCH;
     constexpr int HRS = hrs16_of(LTF);
     constexpr long HSCB = (long)A * LTF * 4;          // channel bytes per subcarrier
@@ -2032,7 +2040,9 @@ int build_fused_params(const aerial_cell_desc* cells, int nCells, FusedParams& p
         }
         p.stageBytes = (b + 15) & ~15;
     }
-    p.nStages = p.exactChunks ? stages_of_a(p.exactTile, p.exactChunks) : stages_of(p.exactTile);
+    p.nStages = !p.exactChunks                 ? stages_of(p.exactTile)
+                : p.fmt == AERIAL_FMT_CF16 ? stages_of_h(p.exactTile, p.exactChunks)
+                                               : stages_of_a(p.exactTile, p.exactChunks);
     warpBytes = p.epiBytes + p.nStages * p.stageBytes;
     return AERIAL_OK;
 }
