@@ -1912,14 +1912,20 @@ namespace aeq {
 // lanes of the solve idle and pays only while half the warps are free (one
 // slot of 132 x 64 x 8: 10.9 us at 1, 10.3 us at 2).
 // A subcarrier's results do not depend on its group.
+// In rounds, three subcarriers of 8 full layers become four, which fill the lanes of
+// their solve: 12 / 24 / 48 uneven cells 40 -> 37, 51 -> 49 and 113 -> 107 us;
+// not with split operands, whose items cost more (24 uneven cells, BF16X3: 57
+// and 58 us).
 constexpr int kMaxItems = 16, kRoundItems = 12;
 
-static long assign_groups(FusedParams& p, int items, int fixed, int cap) {
+// Groups of `fixed` subcarriers, or of about `items` items (fill: see above).
+static long assign_groups(FusedParams& p, int items, int fixed, int cap, bool fill = false) {
     long g0 = 0;
     for (int i = 0; i < p.nCells; i++) {
         FusedCell& f = p.cell[i];
         const int most = 32 / f.LT < cap ? 32 / f.LT : cap;
-        const int gs = fixed ? fixed : (items + f.nChunk / 2) / f.nChunk;
+        int gs = fixed ? fixed : (items + f.nChunk / 2) / f.nChunk;
+        if (fill && f.exact && gs == 3 && f.LT == 8) gs = 4;
         f.GS = gs < 1 ? 1 : gs > most ? most : gs;
         f.group0 = g0;
         g0 += (f.nSC + f.GS - 1) / f.GS;
@@ -1928,7 +1934,7 @@ static long assign_groups(FusedParams& p, int items, int fixed, int cap) {
     return g0;
 }
 
-void set_groups(FusedParams& p, int cap, long warps) {
+void set_groups(FusedParams& p, int cap, long warps, int prec) {
     if (p.exactChunks) {                              // uniform batch
         if (cap < 1) cap = kUniformGroupCap;
         for (int gs = 1; gs < cap; gs *= 2)
@@ -1942,7 +1948,7 @@ void set_groups(FusedParams& p, int cap, long warps) {
     if (subcarriers <= warps * cap)                   // else no grouping fits one round
         for (int items : {1, 2, 3, 4, 5, 6, 8, 10, 12, kMaxItems})
             if (assign_groups(p, items, 0, cap) <= warps) return;
-    assign_groups(p, kRoundItems, 0, cap);
+    assign_groups(p, kRoundItems, 0, cap, prec == AERIAL_PREC_FP16 || prec == AERIAL_PREC_BF16);
 }
 
 // warpBytes: the per-warp shared memory of the launch (epilogue region of the
@@ -2394,7 +2400,7 @@ extern "C" int aerial_pusch_eq_fused(const aerial_cell_desc* cells, int nCells, 
     LaunchShape sh;
     int prec, gsCap;
     resolve_tuning(tuning, warpBytes, prec, sh, gsCap);
-    set_groups(p, gsCap, resident_warps(sh));
+    set_groups(p, gsCap, resident_warps(sh), prec);
     set_operand_scale(p, prec);
     return launch_fused(p, warpBytes, prec, sh, to_stream(stream));
 }
@@ -2455,7 +2461,7 @@ extern "C" int aerial_autotune(const aerial_cell_desc* cells, int nCells, aerial
         for (int ic = 0; ic < nc && !s; ic++) {
             const LaunchShape& sh = cand[ic].sh;
             p = base;                                // unscaled sigma2
-            set_groups(p, cand[ic].cap, resident_warps(sh));
+            set_groups(p, cand[ic].cap, resident_warps(sh), prec);
             set_operand_scale(p, prec);
             if ((s = launch_fused(p, warpBytes, prec, sh, st))) break;
             cudaEventRecord(e0, st);
@@ -2547,7 +2553,7 @@ extern "C" int aerial_eq_graph_create(const aerial_cell_desc* cells, int nCells,
     int s = build_fused_params(cells, nCells, g->params, warpBytes);
     if (!s) {
         resolve_tuning(tuning, warpBytes, g->prec, g->shape, g->gsCap);
-        set_groups(g->params, g->gsCap, resident_warps(g->shape));
+        set_groups(g->params, g->gsCap, resident_warps(g->shape), g->prec);
         set_operand_scale(g->params, g->prec);
         s = plan_fused(g->params, warpBytes, g->prec, g->shape, g->plan);
     }
@@ -2600,7 +2606,7 @@ extern "C" int aerial_eq_graph_update(aerial_eq_graph* g, const aerial_cell_desc
     // The new noise levels may move a cell in or out of FP16 operand scaling,
     // which selects another kernel instantiation: re-plan the node (an
     // executable graph's kernel node may change its function).
-    set_groups(np, g->gsCap, resident_warps(g->shape));
+    set_groups(np, g->gsCap, resident_warps(g->shape), g->prec);
     set_operand_scale(np, g->prec);
     np.walkSlot = g->params.walkSlot;
     LaunchPlan pl;
