@@ -41,8 +41,8 @@ __device__ __forceinline__ float4 ld_pair(const float2* p, int a0, int A, bool i
 // k-steps whose loads are issued together.  The kernel is bound by the bytes
 // it has in flight: one k-step's three 16-byte loads a lane before their MMAs
 // left HBM at 4.2 TB/s.  8 slots of 1,584 subcarriers, 64 antennas, 8 layers,
-// 14 symbols (154 MB): 37 -> 26 us.
-constexpr int kTcSteps = 4;
+// 14 symbols (154 MB): 37 us, 30 us with four k-steps at a time, 27 us with eight.
+constexpr int kTcSteps = 8;
 
 // NMT, NNT: 8-layer and 8-symbol tiles.
 template <int NMT, int NNT, bool VEC>

@@ -552,11 +552,11 @@ __global__ void __launch_bounds__(kGramThreads) gram_kernel(const GramParams p) 
 // one store as wide as they are (32 bytes of 256-QAM in FP32 fill a sector;
 // as four 8-byte stores each of a warp's requests left every sector of 1 KB a
 // quarter full).  14-symbol 256-QAM of 8 slots of 1,584 subcarriers x 8
-// layers, 57 MB: 21.5 -> 12 us.  64-QAM rows (24 bytes) cross through shared
+// layers, 57 MB: 21.5 -> 10 us.  64-QAM rows (24 bytes) cross through shared
 // memory into 16-byte stores.  Less aligned outputs take the narrow stores.
 // ---------------------------------------------------------------------------
-constexpr int kLlrThreads = 512;
-constexpr int kLlrPerThread = 2;               // symbols a thread loads before it demaps the first
+constexpr int kLlrThreads = 256;
+constexpr int kLlrPerThread = 4;               // symbols a thread loads before it demaps the first
 
 // W: 4-byte words of LLRs per symbol.
 template <int W>
@@ -573,7 +573,7 @@ __device__ __forceinline__ void store_words(uint32_t* dst, const uint32_t (&v)[W
         *dst = v[0];
 }
 
-// The block's symbols base .. base + 511 (count in all).  wide: out is aligned
+// The block's symbols base .. base + 255 (count in all).  wide: out is aligned
 // to the row's store (16 bytes for rows of 3 or 6 words); otherwise NARROW
 // words at a time (FP32 LLR rows are 8-byte aligned, FP16 ones 4-byte).
 template <int W, int NARROW>
