@@ -25,15 +25,19 @@ __device__ __forceinline__ void mma_f16(float* d, uint32_t a0, uint32_t a1, uint
 }
 
 // The pair p[a0], p[a0 + 1] of a row of A values; zeros for a row that does
-// not exist (in = false) and past the row's end.
+// not exist (in = false) and past the row's end.  Ordinary and volatile loads
+// (wait_previous): C and Y are what earlier kernels of the stream wrote.
 template <bool VEC>
 __device__ __forceinline__ float4 ld_pair(const float2* p, int a0, int A, bool in) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (VEC) {                         // A even, 16-byte rows
-        if (in && a0 < A) v = __ldcs(reinterpret_cast<const float4*>(p + a0));
+        if (in && a0 < A)
+            asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                         : "l"(__cvta_generic_to_global(p + a0)));
     } else {
-        if (in && a0 < A) { const float2 t = __ldg(p + a0); v.x = t.x; v.y = t.y; }
-        if (in && a0 + 1 < A) { const float2 t = __ldg(p + a0 + 1); v.z = t.x; v.w = t.y; }
+        if (in && a0 < A) { const float2 t = p[a0]; v.x = t.x; v.y = t.y; }
+        if (in && a0 + 1 < A) { const float2 t = p[a0 + 1]; v.z = t.x; v.w = t.y; }
     }
     return v;
 }
@@ -46,8 +50,7 @@ constexpr int kTcSteps = 8;
 
 // NMT, NNT: 8-layer and 8-symbol tiles.
 template <int NMT, int NNT, bool VEC>
-__global__ void __launch_bounds__(256) coef_apply_tc_kernel(const float2* __restrict__ C, const float2* __restrict__ Y,
-                                                             float2* __restrict__ O, int nSC, int nSym, int L, int A) {
+__global__ void __launch_bounds__(256) coef_apply_tc_kernel(const float2* C, const float2* Y, float2* O, int nSC, int nSym, int L, int A) {
     wait_previous();
     const int lane = threadIdx.x & 31;
     const int g = lane >> 2, c = lane & 3;

@@ -108,7 +108,10 @@ int allow_max_smem() {
 // kernel of its stream has finished, before that kernel's writes are flushed and
 // its completion is known.  Every kernel so launched calls wait_previous before
 // it touches memory: it returns once the earlier kernels of the stream have
-// completed and their writes are visible (at once if there are none).  Back to
+// completed and their writes are visible (at once if there are none).  What an
+// earlier kernel may have written is read by ordinary loads, which the compiler
+// keeps behind the wait, or by volatile asm: never through the read-only path
+// (const __restrict__ pointers, __ldg) or a cache-hint intrinsic.  Back to
 // back, plain launches -> these: one slot of 132 PRB x 64 antennas x 8 layers
 // 8.2 -> 6.6 us, 12 ragged cells 22.5 -> 20.6, Gram + coef_apply + demapper of 8
 // slots 62.7 -> 58.1 us.  Letting the next kernel's blocks in while this one's

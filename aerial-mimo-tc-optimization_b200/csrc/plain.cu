@@ -605,10 +605,8 @@ __device__ __forceinline__ void write_rows(uint32_t* out, long base, int count, 
 }
 
 template <int N>
-__global__ void __launch_bounds__(kLlrThreads) llr_f16_kernel(const __half2* __restrict__ in,
-                                                               const float* __restrict__ ni,
-                                                               __half* __restrict__ out, int count, bool wide,
-                                                               PamLut lut) {
+__global__ void __launch_bounds__(kLlrThreads) llr_f16_kernel(const __half2* in, const float* ni, __half* out, int count,
+                                                               bool wide, PamLut lut) {
     wait_previous();
     __half2 v[kLlrPerThread];
     float nv[kLlrPerThread];
@@ -637,10 +635,8 @@ __global__ void __launch_bounds__(kLlrThreads) llr_f16_kernel(const __half2* __r
 // division, the rest from it (rcp = floor(2^32 / symsPerNoise) + 1, exact
 // while symsPerNoise <= 1024; a larger count changes at most once in a block).
 template <int N>
-__global__ void __launch_bounds__(kLlrThreads) llr_f32_kernel(const cf* __restrict__ in,
-                                                               const float* __restrict__ ni,
-                                                               float* __restrict__ out, int count, int symsPerNoise,
-                                                               unsigned rcp, bool wide, PamLut lut) {
+__global__ void __launch_bounds__(kLlrThreads) llr_f32_kernel(const cf* in, const float* ni, float* out, int count,
+                                                               int symsPerNoise, unsigned rcp, bool wide, PamLut lut) {
     wait_previous();
     cf v[kLlrPerThread];
     float nv[kLlrPerThread];

@@ -85,10 +85,8 @@ __device__ __forceinline__ void split_h2(float x, float y, uint32_t& hi, uint32_
 // Grid: x = CTAs walking the (block, 16 MT-antenna) items, y = slices of NQ
 // output groups (16 complex outputs per group).
 template <int KS, int MT, int OUTL>
-__global__ void __launch_bounds__(kSrsWarps * 32, 2) srs_filter_tc_kernel(const __half2* __restrict__ srs,
-                                                                          const __half2* __restrict__ W,
-                                                                          const __half2* __restrict__ focc,
-                                                                          void* __restrict__ out, int nAnt,
+__global__ void __launch_bounds__(kSrsWarps * 32, 2) srs_filter_tc_kernel(const __half2* srs, const __half2* W,
+                                                                          const __half2* focc, void* out, int nAnt,
                                                                           int nBlocks, int K, int Ko, int P, int F, int NQ) {
     wait_previous();
     extern __shared__ uint4 bfrag[];            // [group][kstep][tile][lane]: {b0 hi, b1 hi, b0 lo, b1 lo}
@@ -145,12 +143,12 @@ __global__ void __launch_bounds__(kSrsWarps * 32, 2) srs_filter_tc_kernel(const 
                     uint32_t v0 = 0u, v1 = 0u;
                     if (av && k < K) {
                         if (pairK) {
-                            const uint2 v = __ldg(reinterpret_cast<const uint2*>(row + k));
+                            const uint2 v = *reinterpret_cast<const uint2*>(row + k);
                             v0 = v.x;
                             v1 = v.y;
                         } else {
-                            v0 = h2bits(__ldg(row + k));
-                            if (k + 1 < K) v1 = h2bits(__ldg(row + k + 1));
+                            v0 = h2bits(row[k]);
+                            if (k + 1 < K) v1 = h2bits(row[k + 1]);
                         }
                     }
                     a[mt][ks][rr] = v0;
@@ -336,10 +334,9 @@ __device__ __forceinline__ uint32_t sw128_off(int r, int k) {
 // these counts), so (1/S) sum_s f(in_s) is one GEMM with K extended over S.
 template <int KB, int NTL, int OUTL>
 __global__ void __launch_bounds__(kUmmaThreads, 1) chest_umma_kernel(const __grid_constant__ CUtensorMap tmA,
-                                                                      const __half2* __restrict__ Wf,
-                                                                      const __half2* __restrict__ occ,
-                                                                      void* __restrict__ out, int nAnt, int nBlocks,
-                                                                      int nPilot, int nOut, int P, int F, int nSrs) {
+                                                                      const __half2* Wf, const __half2* occ, void* out,
+                                                                      int nAnt, int nBlocks, int nPilot, int nOut, int P,
+                                                                      int F, int nSrs) {
     extern __shared__ __align__(1024) uint8_t usm_raw[];
     wait_previous();
     // 128-byte swizzle atoms must start on 1024-byte boundaries of the shared window
