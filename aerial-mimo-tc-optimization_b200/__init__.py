@@ -347,7 +347,8 @@ def pusch_eq_plain_workspace(cells) -> int:
 
 
 def pusch_eq_plain(cells, workspace, stream=None):
-    """The plain FP32 chain (gram, mmse_coef, coef_apply, llr_f32 of each cell, in one kernel)."""
+    """The plain FP32 chain (gram, mmse_coef, coef_apply, llr_f32 of each cell in order; one kernel
+    for consecutive cells unless their buffers overlap)."""
     arr, n = _cells_array(cells)
     _check(lib().aerial_pusch_eq_plain(arr, n, _ptr(workspace), workspace.numel() * workspace.element_size(),
                                        _stream(stream)), "pusch_eq_plain")

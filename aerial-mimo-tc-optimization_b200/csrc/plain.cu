@@ -797,6 +797,8 @@ static int launch_llr_f32(const cf* in, const float* ni, float* out, int N, int 
 
 namespace aeq {
 
+int static_scratch(char** out);
+
 // Load the plain chain's kernels on the current device (aerial_prepare).
 template <typename K>
 static int prepare_one(K* k) {
@@ -890,21 +892,28 @@ extern "C" int aerial_llr_f32(const aerial_cf32* softEst, const float* noiseInv,
 }
 
 // ---------------------------------------------------------------------------
-// The plain chain over cells.  The workspace (G, C, noiseInv and Y_eq of the
-// largest cell) is part of the interface and checked; the chain's kernel keeps
-// them on chip and does not touch it.
+// The plain chain over cells.  The chain's kernel keeps G, C and noiseInv on
+// chip; the workspace (these and Y_eq of the largest cell) is part of the
+// interface, checked, and used where a cell has to run stage by stage.
 // ---------------------------------------------------------------------------
-static size_t plain_ws_cell(const aerial_cell_desc& c) {
+struct PlainWs {
+    size_t C, nInv, yeq, total;        // offsets; G comes first
+};
+static PlainWs plain_ws_cell(const aerial_cell_desc& c) {
     size_t nSC = (size_t)c.nPRB * 12;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    return al(nSC * c.nLayers * c.nLayers * sizeof(cf)) + al(nSC * c.nLayers * c.nAnt * sizeof(cf)) +
-           al(nSC * c.nLayers * sizeof(float)) + al(nSC * c.nLayers * c.nSym * sizeof(cf));
+    PlainWs w;
+    w.C = al(nSC * c.nLayers * c.nLayers * sizeof(cf));
+    w.nInv = w.C + al(nSC * c.nLayers * c.nAnt * sizeof(cf));
+    w.yeq = w.nInv + al(nSC * c.nLayers * sizeof(float));
+    w.total = w.yeq + al(nSC * c.nLayers * c.nSym * sizeof(cf));
+    return w;
 }
 
 extern "C" size_t aerial_pusch_eq_plain_workspace(const aerial_cell_desc* cells, int nCells) {
     size_t m = 0;
     for (int i = 0; cells && i < nCells; i++) {
-        size_t w = plain_ws_cell(cells[i]);
+        size_t w = plain_ws_cell(cells[i]).total;
         if (w > m) m = w;
     }
     return m;
@@ -920,19 +929,71 @@ static int plain_cell_check(const aerial_cell_desc& c) {
     return AERIAL_OK;
 }
 
-// Consecutive cells whose layers share a tile go into one launch; the chain
-// needs no memory of its own.
-static int run_plain(const aerial_cell_desc* cells, int nCells, cudaStream_t st) {
+// A cell's buffers.  The specification runs the cells of a call in order, and
+// each cell stage by stage, so a later cell may use what an earlier one wrote or
+// write over what it is done with, and a cell's outputs may lie over inputs that
+// its earlier stages have read.  The kernel runs all its subcarriers at once.
+struct PlainBuffers {
+    uintptr_t in[2], inEnd[2], out[2], outEnd[2];
+};
+static PlainBuffers plain_buffers(const aerial_cell_desc& c) {
+    const size_t nSC = (size_t)c.nPRB * 12, res = nSC * c.nLayers * c.nSym;
+    PlainBuffers b;
+    b.in[0] = (uintptr_t)c.H;
+    b.inEnd[0] = b.in[0] + nSC * c.nAnt * c.nLayers * sizeof(cf);
+    b.in[1] = (uintptr_t)c.Y_rx;
+    b.inEnd[1] = b.in[1] + nSC * c.nSym * c.nAnt * sizeof(cf);
+    b.out[0] = (uintptr_t)c.llr;
+    b.outEnd[0] = b.out[0] + res * 2 * c.nPamBits * sizeof(float);
+    b.out[1] = (uintptr_t)c.Y_eq;
+    b.outEnd[1] = c.Y_eq ? b.out[1] + res * sizeof(cf) : b.out[1];
+    return b;
+}
+// Whether a buffer that `a` writes overlaps one that `b` reads, or (outs) writes.
+static bool plain_touches(const PlainBuffers& a, const PlainBuffers& b, bool outs) {
+    for (int i = 0; i < 2; i++)
+        for (int j = 0; j < 2; j++)
+            if ((a.out[i] < b.inEnd[j] && b.in[j] < a.outEnd[i]) ||
+                (outs && a.out[i] < b.outEnd[j] && b.out[j] < a.outEnd[i]))
+                return true;
+    return false;
+}
+
+static int run_staged(const aerial_cell_desc& c, char* ws, cudaStream_t st) {
+    const PlainWs w = plain_ws_cell(c);
+    const int nSC = c.nPRB * 12;
+    const cf* H = (const cf*)c.H;
+    cf *G = (cf*)ws, *C = (cf*)(ws + w.C), *yeq = c.Y_eq ? (cf*)c.Y_eq : (cf*)(ws + w.yeq);
+    float* nInv = (float*)(ws + w.nInv);
+    int s = launch_gram(H, c.sigma2, G, nSC, c.nAnt, c.nLayers, st);
+    if (!s) s = launch_mmse_coef(G, H, C, nInv, nSC, c.nAnt, c.nLayers, st);
+    if (!s) s = launch_coef_apply(C, (const cf*)c.Y_rx, yeq, nSC, c.nSym, c.nLayers, c.nAnt, st);
+    return s ? s : launch_llr_f32(yeq, nInv, c.llr, nSC * c.nLayers * c.nSym, c.nPamBits, c.nSym, st);
+}
+
+// Consecutive cells whose layers share a tile and whose buffers are independent
+// go into one launch; a cell whose outputs overlap its own inputs runs stage by
+// stage in the workspace.
+static int run_plain(const aerial_cell_desc* cells, int nCells, char* ws, cudaStream_t st) {
+    PlainBuffers held[AERIAL_MAX_CELLS];
     for (int i = 0; i < nCells;) {
         PlainParams p;
         p.nCells = 0;
         const int tile = layers_tile(cells[i].nLayers);
         long subcarriers = 0;                        // block indices stay in 31 bits
+        bool staged = false;
         for (; i < nCells && p.nCells < AERIAL_MAX_CELLS && layers_tile(cells[i].nLayers) == tile; i++) {
             const aerial_cell_desc& c = cells[i];
             const int nSC = c.nPRB * 12;
             if (p.nCells && subcarriers + nSC > INT32_MAX / 2) break;
+            const PlainBuffers b = plain_buffers(c);
+            bool apart = !plain_touches(b, b, false);
+            staged = !apart && !p.nCells;
+            for (int j = 0; j < p.nCells && apart; j++)
+                apart = !plain_touches(held[j], b, true) && !plain_touches(b, held[j], false);
+            if (!apart) break;
             subcarriers += nSC;
+            held[p.nCells] = b;
             PlainCell& d = p.cell[p.nCells++];
             d = plain_cell((const cf*)c.H, (const cf*)c.Y_rx, nSC, c.nAnt, c.nLayers, c.nSym);
             d.O = (cf*)c.Y_eq;
@@ -941,7 +1002,7 @@ static int run_plain(const aerial_cell_desc* cells, int nCells, cudaStream_t st)
             d.nPam = c.nPamBits;
             d.lut = pam_lut(c.nPamBits);
         }
-        const int s = launch_plain<kChain>(p, st);
+        const int s = staged ? run_staged(cells[i++], ws, st) : launch_plain<kChain>(p, st);
         if (s) return s;
     }
     return AERIAL_OK;
@@ -953,9 +1014,9 @@ extern "C" int aerial_pusch_eq_plain(const aerial_cell_desc* cells, int nCells, 
     for (int i = 0; i < nCells; i++) {
         const int s = plain_cell_check(cells[i]);
         if (s != AERIAL_OK) return s;
-        if (plain_ws_cell(cells[i]) > wsBytes) return AERIAL_ERR_INVALID_ARG;
+        if (plain_ws_cell(cells[i]).total > wsBytes) return AERIAL_ERR_INVALID_ARG;
     }
-    return run_plain(cells, nCells, to_stream(stream));
+    return run_plain(cells, nCells, static_cast<char*>(workspace), to_stream(stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -966,7 +1027,8 @@ extern "C" int aerial_pusch_eq_plain(const aerial_cell_desc* cells, int nCells, 
 // device and miss the slot deadline, or a plugin inside a framework that owns
 // all device memory and hands out none.  The chain's intermediates (G, C,
 // noiseInv) live in shared memory, so this entry point needs no device memory
-// at all; a batch whose largest cell's intermediates would exceed
+// but for a cell that has to run stage by stage, which takes the library's static
+// scratch; a batch whose largest cell's intermediates would exceed its
 // AERIAL_STATIC_SCRATCH_BYTES is refused, as the interface states.
 // ---------------------------------------------------------------------------
 extern "C" int aerial_pusch_eq_plain_static(const aerial_cell_desc* cells, int nCells, void* stream) {
@@ -977,5 +1039,12 @@ extern "C" int aerial_pusch_eq_plain_static(const aerial_cell_desc* cells, int n
     }
     if (aerial_pusch_eq_plain_workspace(cells, nCells) > (size_t)AERIAL_STATIC_SCRATCH_BYTES)
         return AERIAL_ERR_SCRATCH_LIMIT;
-    return run_plain(cells, nCells, to_stream(stream));
+    char* ws = nullptr;
+    for (int i = 0; i < nCells && !ws; i++) {
+        const PlainBuffers b = plain_buffers(cells[i]);
+        if (!plain_touches(b, b, false)) continue;
+        const int s = static_scratch(&ws);
+        if (s != AERIAL_OK) return s;
+    }
+    return run_plain(cells, nCells, ws, to_stream(stream));
 }

@@ -312,10 +312,14 @@ int aerial_pusch_eq_host(const aerial_cell_desc* cells, int nCells, const aerial
 
 /* The plain FP32 chain for the same cells: the results of aerial_gram,
  * aerial_mmse_coef, aerial_coef_apply and aerial_llr_f32 per cell, bit for bit,
- * which is the reference's stage-by-stage scalar method on the GPU.  One kernel
- * runs all stages with the intermediates on chip; the workspace (size from
- * aerial_pusch_eq_plain_workspace) is checked and left as it is.  Every cell
- * is checked before anything is launched. */
+ * which is the reference's stage-by-stage scalar method on the GPU.  Every cell
+ * is checked before anything is launched.  One kernel runs all stages of
+ * consecutive cells with the intermediates on chip.  The results are those of
+ * the cells in order, stage by stage: a cell may read or overwrite the buffers
+ * of the cells before it (it then goes into a launch of its own), and its llr
+ * may lie over its H or Y_rx and its Y_eq over its H (the cell then runs as
+ * separate stages).  The workspace (size from aerial_pusch_eq_plain_workspace)
+ * is written in that last case only. */
 size_t aerial_pusch_eq_plain_workspace(const aerial_cell_desc* cells, int nCells);
 int aerial_pusch_eq_plain(const aerial_cell_desc* cells, int nCells, void* workspace,
                           size_t workspaceBytes, void* stream);
@@ -324,13 +328,16 @@ int aerial_pusch_eq_plain(const aerial_cell_desc* cells, int nCells, void* works
  * real-time slot loop where cudaMalloc may block or synchronize the device,
  * or a plugin whose host framework owns all device memory.  No counterpart in
  * the reference.  Same cells and results as aerial_pusch_eq_plain, with no
- * device memory but the cells' own; calls may overlap on the GPU.  A batch
- * whose largest cell has intermediates of more than
- * AERIAL_STATIC_SCRATCH_BYTES (16 MiB; see aerial_pusch_eq_plain_workspace;
- * e.g. a 273-PRB, 128-antenna, 16-layer cell) is rejected with
- * AERIAL_ERR_SCRATCH_LIMIT before anything runs.  Malformed cells return
- * AERIAL_ERR_INVALID_ARG (or AERIAL_ERR_UNSUPPORTED for a complex-half cell)
- * before the size check. */
+ * device memory but the cells' own, except that a cell whose llr or Y_eq
+ * overlaps its own H or Y_rx runs its stages in a static array of the
+ * library's, which the first call with such a cell in a CUDA context loads
+ * (make it before any stream capture) and which all such calls share.  Other
+ * calls may overlap on the GPU.  A batch whose largest cell has intermediates
+ * of more than AERIAL_STATIC_SCRATCH_BYTES (16 MiB; see
+ * aerial_pusch_eq_plain_workspace; e.g. a 273-PRB, 128-antenna, 16-layer cell)
+ * is rejected with AERIAL_ERR_SCRATCH_LIMIT before anything runs.  Malformed
+ * cells return AERIAL_ERR_INVALID_ARG (or AERIAL_ERR_UNSUPPORTED for a
+ * complex-half cell) before the size check. */
 #define AERIAL_STATIC_SCRATCH_BYTES (16u << 20)
 int aerial_pusch_eq_plain_static(const aerial_cell_desc* cells, int nCells, void* stream);
 
