@@ -86,20 +86,22 @@ inline int sm_count() {
     return n;
 }
 
-// Raises kernel K's dynamic shared-memory limit to the per-block maximum,
-// once per device (the launch's own request then sets its occupancy).
+// Raises kernel K's dynamic shared-memory limit to the per-block maximum (the
+// launch's own request then sets its occupancy).  The limit belongs to the
+// kernel as loaded in one context: it is set when the device's current context is
+// another than at the last call (a second context, or one after a device reset).
 template <auto K>
 int allow_max_smem() {
-    static std::mutex mu;
-    static bool done[kMaxDevices] = {};
+    static std::atomic<unsigned long long> done[kMaxDevices];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return rt_status(e);
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev >= 0 && dev < kMaxDevices && done[dev]) return AERIAL_OK;
+    const bool cached = dev >= 0 && dev < kMaxDevices;
+    const unsigned long long ctx = current_ctx_id();
+    if (cached && ctx != 0 && done[dev].load(std::memory_order_acquire) == ctx) return AERIAL_OK;
     e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemPerCta);
     if (e != cudaSuccess) return rt_status(e);
-    if (dev >= 0 && dev < kMaxDevices) done[dev] = true;
+    if (cached) done[dev].store(current_ctx_id(), std::memory_order_release);   // the call may have made the context
     return AERIAL_OK;
 }
 
