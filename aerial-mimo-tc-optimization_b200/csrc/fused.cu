@@ -27,6 +27,7 @@
 // n-tile B = H, i.e. the same registers as A.  Thread (g = lane/4, c = lane%4)
 // covers antennas 8j+2c and 8j+2c+1 of k-step j (the K order is permuted
 // inside each k-step; A and B use the same permutation).
+#include <algorithm>
 #include <cstdlib>
 #include <type_traits>
 
@@ -39,11 +40,12 @@ constexpr int kMaxCells = AERIAL_MAX_CELLS;
 // Subcarriers per group (set_groups): at most 32 / LT, which fills every lane
 // of the FP32 solve and of the LLR epilogue (LT lanes per subcarrier), and at
 // most a cap: aerial_tuning.sc_per_group, searched by the autotuner, or these
-// where it is 0.  The uniform batches' kernels hand out groups dynamically
+// where it is 0.  kFullGroups, which caps no tile, asks for full groups.  The uniform batches' kernels hand out groups dynamically
 // and run best with the solve's lanes full at 8 layers and short groups below
 // (16 cells of 273 PRB, 4 layers, 64 antennas: 85 us at 4, 93 us at 8).
 constexpr int kUniformGroupCap = 4;
 constexpr int kMixedGroupCap = 8;
+constexpr int kFullGroups = 32;
 
 struct FusedCell {
     const float2* H;
@@ -1935,6 +1937,10 @@ static long assign_groups(FusedParams& p, int items, int fixed, int cap, bool fi
 }
 
 void set_groups(FusedParams& p, int cap, long warps, int prec) {
+    if (cap >= kFullGroups) {
+        assign_groups(p, 0, kFullGroups, kFullGroups);
+        return;
+    }
     if (p.exactChunks) {                              // uniform batch
         if (cap < 1) cap = kUniformGroupCap;
         for (int gs = 1; gs < cap; gs *= 2)
@@ -2407,11 +2413,12 @@ extern "C" int aerial_pusch_eq_fused(const aerial_cell_desc* cells, int nCells, 
 
 // ---------------------------------------------------------------------------
 // Autotuner: time each candidate tile and launch shape on the caller's cells
-// and keep the fastest.  Candidates are the group cap (most subcarriers solved
-// together per warp: 4, 8 or 32, for batches with tiles of 4 layers or fewer,
-// where the cap changes anything) crossed with (warps per CTA, CTAs per SM)
-// pairs whose shared memory fits one SM; each is timed with CUDA events over
-// a few launches after one warm-up launch.  The reference's analogue is its
+// and keep the fastest.  Candidates are (warps per CTA, CTAs per SM) pairs whose
+// shared memory fits one SM crossed with the group cap (aerial_tuning.
+// sc_per_group: the default one and, for batches with tiles of 4 layers or
+// fewer, the other of 4 and 8, and full groups), less the caps that group the
+// batch as an earlier one does; each is timed with CUDA events over a few
+// launches after one warm-up launch.  The reference's analogue is its
 // templated shape sweep over antennas and symbols (src/coef_scaling.cu:221-250).
 // ---------------------------------------------------------------------------
 extern "C" int aerial_autotune(const aerial_cell_desc* cells, int nCells, aerial_tuning* best, float* bestUs,
@@ -2427,26 +2434,33 @@ extern "C" int aerial_autotune(const aerial_cell_desc* cells, int nCells, aerial
         LaunchShape sh;
         int cap;
     };
-    int caps[3] = {kUniformGroupCap, 0, 0}, nCaps = 1;
-    bool smallTile = false;
-    for (int i = 0; i < base.nCells; i++) smallTile |= base.cell[i].LT <= 4;
-    if (smallTile) {
-        caps[nCaps++] = 8;
-        caps[nCaps++] = 32;
-    }
+    const int defCap = base.exactChunks ? kUniformGroupCap : kMixedGroupCap;
+    const int caps[3] = {defCap, kUniformGroupCap + kMixedGroupCap - defCap, kFullGroups};
+    int nCaps = 1;
+    for (int i = 0; i < base.nCells; i++)
+        if (base.cell[i].LT <= 4) nCaps = 3;
     Cand cand[48];
     int nc = 0;
     const LaunchShape def = default_shape(warpBytes);
-    for (int ic = 0; ic < nCaps; ic++) {
-        bool hasDef = false;
-        for (int w : {2, 3, 4, 6, 8}) {
-            const int k = max_ctas(w, warpBytes);
-            if (k >= 1) cand[nc++] = {{w, k}, caps[ic]};
-            if (k >= 2) cand[nc++] = {{w, k - 1}, caps[ic]};
-            hasDef |= w == def.warps && ((k >= 1 && k == def.ctasPerSm) || (k >= 2 && k - 1 == def.ctasPerSm));
+    auto add = [&](LaunchShape sh) {
+        int gs[3][kMaxCells];
+        for (int ic = 0; ic < nCaps; ic++) {
+            p = base;
+            set_groups(p, caps[ic], resident_warps(sh), prec);
+            bool seen = false;
+            for (int i = 0; i < p.nCells; i++) gs[ic][i] = p.cell[i].GS;
+            for (int k = 0; k < ic && !seen; k++) seen = std::equal(gs[k], gs[k] + p.nCells, gs[ic]);
+            if (!seen) cand[nc++] = {sh, caps[ic]};
         }
-        if (!hasDef) cand[nc++] = {def, caps[ic]};
+    };
+    bool hasDef = false;
+    for (int w : {2, 3, 4, 6, 8}) {
+        const int k = max_ctas(w, warpBytes);
+        if (k >= 1) add({w, k});
+        if (k >= 2) add({w, k - 1});
+        hasDef |= w == def.warps && ((k >= 1 && k == def.ctasPerSm) || (k >= 2 && k - 1 == def.ctasPerSm));
     }
+    if (!hasDef) add(def);
     // Rounds interleave the candidates so clock drift under the power cap
     // hits all of them alike; a candidate's time is its best round.  Within
     // 2 % of the fastest, the shape with more resident warps wins (it holds
@@ -2481,14 +2495,14 @@ extern "C" int aerial_autotune(const aerial_cell_desc* cells, int nCells, aerial
     }
     float fastest = 1e30f;
     for (int ic = 0; ic < nc; ic++) fastest = t[ic] < fastest ? t[ic] : fastest;
-    Cand bestC{def, kUniformGroupCap};
+    Cand bestC{def, defCap};
     float bestT = 1e30f;
     int bestWarps = -1;
     for (int ic = 0; ic < nc; ic++) {
         if (t[ic] > fastest * 1.02f) continue;
         const int w = cand[ic].sh.warps * cand[ic].sh.ctasPerSm;
         const bool better = w > bestWarps ||
-                            (w == bestWarps && cand[ic].cap == kUniformGroupCap && bestC.cap != kUniformGroupCap) ||
+                            (w == bestWarps && cand[ic].cap == defCap && bestC.cap != defCap) ||
                             (w == bestWarps && cand[ic].cap == bestC.cap && t[ic] < bestT);
         if (better) {
             bestWarps = w;

@@ -268,7 +268,8 @@ typedef struct {
                                   (at most min(32 / layer tile, cap); fewer
                                   where the launch is small or a cell has many
                                   antennas, so that no warp is left with a few
-                                  long groups); 0 = default (4 for uniform
+                                  long groups); 32 or more: 32 / layer tile
+                                  everywhere; 0 = default (cap 4 for uniform
                                   batches, 8 for mixed ones) */
 } aerial_tuning;
 
