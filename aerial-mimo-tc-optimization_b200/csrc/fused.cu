@@ -1907,17 +1907,25 @@ namespace aeq {
 // one slot of 24 PRB x 32 antennas x 4 layers 8.3 -> 6.3 us, two of
 // 132 x 64 x 8 16.5 -> 14.5, one of 100 PRB x 48 x 3 16.5 -> 10.4; mixed
 // batches of 8 / 16 / 48 cells 32.9 -> 27 / 34 -> 33 / 112 -> 103 us, of 24
-// and 48 cells with ragged shapes 72 -> 53 and 114 -> 106 us.  Over 58 random
-// batches of 1 to 64 cells it is 2 % off the best of 13 item counts (geometric
-// mean), four subcarriers a group 22 %; 8 or 16 items in the rounds' place
-// 3.6 % and 2.8 %.  One subcarrier a group in a uniform batch keeps most
-// lanes of the solve idle and pays only while half the warps are free (one
-// slot of 132 x 64 x 8: 10.9 us at 1, 10.3 us at 2).
+// and 48 cells with ragged shapes 72 -> 53 and 114 -> 106 us.  8 or 16 items in
+// the rounds' place are 1 % slower over mixed batches.  One subcarrier a group
+// in a uniform batch keeps most lanes of the solve idle and pays only while half
+// the warps are free (one slot of 132 x 64 x 8: 10.9 us at 1, 10.3 us at 2).
 // A subcarrier's results do not depend on its group.
+//
 // In rounds, three subcarriers of 8 full layers become four, which fill the lanes of
 // their solve: 12 / 24 / 48 uneven cells 40 -> 37, 51 -> 49 and 113 -> 107 us;
 // not with split operands, whose items cost more (24 uneven cells, BF16X3: 57
 // and 58 us).
+//
+// Cells of one tile and chunk count (outside the uniform kernels) have groups of
+// one length, and what they cost is known better than by an item count: the
+// rounds, half of whose last one is free because fewer warps share the memory,
+// times a group's items, two more for each subcarrier's results and six for
+// the solve.  The size of least cost is 1 % off the best of 1, 2, 3, 4, 6 and 8
+// over 442 such launches, 12 items a group 3.5 % and up to 28 % (32 slots of
+// 132 PRB x 160 antennas x 16 layers 510 us at 1, 420 us at 2; 4 of 132 x 160 x 8
+// with BF16X3 operands 49 and 39 us at 1 and 4), 4 everywhere 13 %.
 constexpr int kMaxItems = 16, kRoundItems = 12;
 
 // Groups of `fixed` subcarriers, or of about `items` items (fill: see above).
@@ -1949,8 +1957,28 @@ void set_groups(FusedParams& p, int cap, long warps, int prec) {
         return;
     }
     if (cap < 1) cap = kMixedGroupCap;
+    const int LT = p.cell[0].LT, nChunk = p.cell[0].nChunk;
+    bool alike = warps > 0;
     long subcarriers = 0;
-    for (int i = 0; i < p.nCells; i++) subcarriers += p.cell[i].nSC;
+    for (int i = 0; i < p.nCells; i++) {
+        subcarriers += p.cell[i].nSC;
+        alike = alike && p.cell[i].LT == LT && p.cell[i].nChunk == nChunk;
+    }
+    if (alike) {
+        int best = 1;
+        double least = 0;
+        for (int gs : {1, 2, 3, 4, 6}) {
+            if (gs > cap || gs > 32 / LT) break;
+            const long groups = assign_groups(p, 0, gs, cap);
+            const double cost = ((groups + warps - 1) / warps + (double)groups / warps) * (gs * (nChunk + 2) + 6);
+            if (gs == 1 || cost < least) {
+                best = gs;
+                least = cost;
+            }
+        }
+        assign_groups(p, 0, best, cap);
+        return;
+    }
     if (subcarriers <= warps * cap)                   // else no grouping fits one round
         for (int items : {1, 2, 3, 4, 5, 6, 8, 10, 12, kMaxItems})
             if (assign_groups(p, items, 0, cap) <= warps) return;
