@@ -1913,10 +1913,10 @@ namespace aeq {
 // the warps are free (one slot of 132 x 64 x 8: 10.9 us at 1, 10.3 us at 2).
 // A subcarrier's results do not depend on its group.
 //
-// In rounds, three subcarriers of 8 full layers become four, which fill the lanes of
-// their solve: 12 / 24 / 48 uneven cells 40 -> 37, 51 -> 49 and 113 -> 107 us;
-// not with split operands, whose items cost more (24 uneven cells, BF16X3: 57
-// and 58 us).
+// In rounds, a group of full layers that leaves a quarter of its solve's lanes
+// idle or less is made a full one (three subcarriers of 8 layers become four):
+// 12 / 24 / 48 uneven cells 40 -> 37, 51 -> 49 and 113 -> 107 us; not with split
+// operands, whose items cost more (24 uneven cells, BF16X3: 57 and 58 us).
 //
 // Cells of one tile and chunk count (outside the uniform kernels) have groups of
 // one length, and what they cost is known better than by an item count: the
@@ -1933,9 +1933,10 @@ static long assign_groups(FusedParams& p, int items, int fixed, int cap, bool fi
     long g0 = 0;
     for (int i = 0; i < p.nCells; i++) {
         FusedCell& f = p.cell[i];
-        const int most = 32 / f.LT < cap ? 32 / f.LT : cap;
+        const int lanes = 32 / f.LT;
+        const int most = lanes < cap ? lanes : cap;
         int gs = fixed ? fixed : (items + f.nChunk / 2) / f.nChunk;
-        if (fill && f.exact && gs == 3 && f.LT == 8) gs = 4;
+        if (fill && f.exact && 4 * gs >= 3 * lanes) gs = lanes;
         f.GS = gs < 1 ? 1 : gs > most ? most : gs;
         f.group0 = g0;
         g0 += (f.nSC + f.GS - 1) / f.GS;
