@@ -451,6 +451,12 @@ __global__ void __launch_bounds__(kPlainThreads) plain_kernel(const __grid_const
 // ---------------------------------------------------------------------------
 constexpr int kGramThreads = 32;
 constexpr int kGramParts = 2;                  // a subcarrier's antennas arrive and are summed in two parts
+// Where a subcarrier's part is at most this many pieces (two for each lane), the
+// lanes walk the pieces of all the warp's subcarriers in one row: taken one
+// subcarrier after another, 16 of them for 1 or 2 layers, a turn with most
+// lanes idle cost as much as a full one.  60 subcarriers x 4 antennas x 1 layer
+// 6.4 us in turns, 1.4 us in one row; x 64 x 2 5.6 and 3.6 us.
+constexpr int kGramFlat = 64;
 __host__ __device__ constexpr int gram_rt(int LT) { return LT == 2 ? 1 : LT == 16 ? 4 : 2; }
 __host__ __device__ constexpr int gram_ct(int LT) { return LT == 16 ? 4 : 2; }
 __host__ __device__ constexpr int gram_team(int LT) { return (LT / gram_rt(LT)) * (LT / gram_ct(LT)); }
@@ -460,25 +466,43 @@ struct GramParams {
     cf* G;
     float sigma2;
     int nSC, A, L, vecH, vecG;
+    // for division of up to 2^16 by the part's antennas and by a row's pieces:
+    // floor(2^32 / d) + 1, or 0 for 1
+    unsigned rcpRows[kGramParts], rcpPieces;
 };
+__device__ __forceinline__ int div_rcp(int v, unsigned rcp) { return rcp ? (int)__umulhi((unsigned)v, rcp) : v; }
+static unsigned rcp_of(int d) { return d > 1 ? (unsigned)(0x100000000ull / (unsigned)d) + 1u : 0u; }
 
 template <int LT, bool EX>
 __global__ void __launch_bounds__(kGramThreads) gram_kernel(const GramParams p) {
     constexpr int RT = gram_rt(LT), CT = gram_ct(LT), TEAM = gram_team(LT), PER = 32 / TEAM;
     extern __shared__ float4 gram_smem[];
     wait_previous();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x;                      // a block is one warp
     const int A = p.A, L = EX ? LT : p.L, hs = EX ? LT + 2 : plain_hs(L);
     const int ts = (A + 1) * hs;                       // values per subcarrier
-    cf* sm = reinterpret_cast<cf*>(gram_smem) + warp * PER * ts;
-    const long sc0 = ((long)blockIdx.x * (blockDim.x >> 5) + warp) * PER;
+    cf* sm = reinterpret_cast<cf*>(gram_smem);
+    const long sc0 = (long)blockIdx.x * PER;
     const int n = (int)min((long)PER, (long)p.nSC - sc0);      // subcarriers of this warp
     const int part = (A + kGramParts - 1) / kGramParts;         // antennas of one copy group
+    const int width = p.vecH ? 2 : 1, pieces = L / width;       // values a copy, copies a row
 #pragma unroll
     for (int q = 0; q < kGramParts; q++) {
         const int a0 = q * part, rows = min(part, A - a0);
-        for (int j = 0; j < n && rows > 0; j++)
-            stage_rows<32, EX ? LT : 0>(sm + j * ts + a0 * hs, hs, p.H + ((sc0 + j) * A + a0) * L, rows, L, p.vecH, lane);
+        if (part * pieces <= kGramFlat) {
+            for (int e = lane; e < n * rows * pieces; e += 32) {
+                const int row = div_rcp(e, p.rcpPieces), k = (e - row * pieces) * width;
+                const int j = div_rcp(row, p.rcpRows[q]), a = a0 + row - j * rows;
+                const cf* src = p.H + ((sc0 + j) * A + a) * L + k;
+                cf* dst = sm + j * ts + a * hs + k;
+                if (p.vecH) cp16(dst, src);
+                else cp8(dst, src);
+            }
+        } else {
+            for (int j = 0; j < n && rows > 0; j++)
+                stage_rows<32, EX ? LT : 0>(sm + j * ts + a0 * hs, hs, p.H + ((sc0 + j) * A + a0) * L, rows, L, p.vecH,
+                                            lane);
+        }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
     const int j = lane / TEAM, t = lane % TEAM;
@@ -735,17 +759,19 @@ template <int LT, bool EX>
 static int launch_gram_t(const GramParams& p, cudaStream_t st) {
     const int s = allow_max_smem<gram_kernel<LT, EX>>();
     if (s) return s;
-    const size_t warpBytes = (size_t)(32 / gram_team(LT)) * (p.A + 1) * plain_hs(p.L) * sizeof(cf);
-    int warps = kGramThreads / 32;
-    while (warps > 1 && warps * warpBytes > (size_t)kMaxSmemPerCta) warps--;   // one warp needs 131 KB at most
-    const long perBlock = (long)warps * (32 / gram_team(LT));
-    const unsigned blocks = (unsigned)((p.nSC + perBlock - 1) / perBlock);
-    return launch_after(gram_kernel<LT, EX>, blocks, warps * 32, warps * warpBytes, st, p);
+    constexpr int PER = 32 / gram_team(LT);
+    // 256 antennas x 16 layers need 131 KB, the most
+    const size_t smem = (size_t)PER * (p.A + 1) * plain_hs(p.L) * sizeof(cf);
+    const unsigned blocks = (unsigned)((p.nSC + PER - 1) / PER);
+    return launch_after(gram_kernel<LT, EX>, blocks, kGramThreads, smem, st, p);
 }
 
 static int launch_gram(const cf* H, float sigma2, cf* G, int nSC, int A, int L, cudaStream_t st) {
     const bool even = (L % 2) == 0;
-    const GramParams p{H, G, sigma2, nSC, A, L, even && ((uintptr_t)H & 15) == 0, even && ((uintptr_t)G & 15) == 0};
+    GramParams p{H, G, sigma2, nSC, A, L, even && ((uintptr_t)H & 15) == 0, even && ((uintptr_t)G & 15) == 0, {}, 0};
+    const int part = (A + kGramParts - 1) / kGramParts;
+    for (int q = 0; q < kGramParts; q++) p.rcpRows[q] = rcp_of(std::min(part, A - q * part));
+    p.rcpPieces = rcp_of(p.vecH ? L / 2 : L);
     switch (layers_tile(L)) {
         case 2: return L == 2 ? launch_gram_t<2, true>(p, st) : launch_gram_t<2, false>(p, st);
         case 4: return L == 4 ? launch_gram_t<4, true>(p, st) : launch_gram_t<4, false>(p, st);
