@@ -571,16 +571,22 @@ __global__ void __launch_bounds__(kGramThreads) gram_kernel(const GramParams p) 
 }
 
 // ---------------------------------------------------------------------------
-// LLR demapper: one thread per symbol (llr_v1_baseline / llr_v3 shape).  It is
-// bound by its writes, 2 N values per symbol read: a thread's LLRs go out in
-// one store as wide as they are (32 bytes of 256-QAM in FP32 fill a sector;
-// as four 8-byte stores each of a warp's requests left every sector of 1 KB a
-// quarter full).  14-symbol 256-QAM of 8 slots of 1,584 subcarriers x 8
-// layers, 57 MB: 21.5 -> 10 us.  64-QAM rows (24 bytes) cross through shared
-// memory into 16-byte stores.  Less aligned outputs take the narrow stores.
+// LLR demapper (llr_v1_baseline / llr_v3 shape), a thread per symbol.  A launch
+// of a block per SM or more is bound by its writes, 2 N values per symbol read:
+// a thread takes four symbols, whose loads are under way together, and a row of
+// LLRs goes out in one store as wide as it is (32 bytes of 256-QAM in FP32 fill a
+// sector; as four 8-byte stores each of a warp's requests left every sector of
+// 1 KB a quarter full).  FP32 rows without such a store, those of 64-QAM (24
+// bytes) and those of 256-QAM in an output that is not aligned for it, cross
+// through shared memory into contiguous stores.  14-symbol 256-QAM of 8 slots of
+// 1,584 subcarriers x 8 layers, 57 MB: 21.5 us with a store per two LLRs, 10 us;
+// 2 M symbols 8 bytes past the alignment 36 us with four stores a symbol, 13.8 us.
+// Smaller launches are bound by one thread's chain, which four symbols and the
+// crossing lengthen: a symbol a thread and direct stores (20,000 symbols of
+// 64-QAM 2.3 us with four, 1.5 us).
 // ---------------------------------------------------------------------------
 constexpr int kLlrThreads = 256;
-constexpr int kLlrPerThread = 4;               // symbols a thread loads before it demaps the first
+constexpr int kLlrSymbols = 4;                 // symbols a thread of a large launch loads before it demaps the first
 
 // W: 4-byte words of LLRs per symbol.
 template <int W>
@@ -597,25 +603,38 @@ __device__ __forceinline__ void store_words(uint32_t* dst, const uint32_t (&v)[W
         *dst = v[0];
 }
 
-// The block's symbols base .. base + 255 (count in all).  wide: out is aligned
-// to the row's store (16 bytes for rows of 3 or 6 words); otherwise NARROW
-// words at a time (FP32 LLR rows are 8-byte aligned, FP16 ones 4-byte).
-template <int W, int NARROW>
+// LLRs of the symbols base .. base + 255 (count in all), a row of W words from
+// each thread.  wide: out is aligned to the row's store, for rows of 6 words to 16
+// bytes; otherwise stores of NARROW words (FP32 LLR rows are 8-byte aligned, FP16
+// ones 4-byte).  CROSS: rows of 24 bytes or more that have no store of their own
+// go by way of shared memory; shorter ones gain nothing there (2 M symbols of
+// 64-QAM in FP16 9.0 us that way, 8.4 us in three direct stores).
+template <int W, int NARROW, bool CROSS>
 __device__ __forceinline__ void write_rows(uint32_t* out, long base, int count, const uint32_t (&v)[W], bool wide) {
     const long idx = base + threadIdx.x;
-    if constexpr (W == 6 || W == 3) {
-        __shared__ __align__(16) uint32_t rows[kLlrThreads * W];
-        if (wide && base + kLlrThreads <= count) {
-#pragma unroll
-            for (int j = 0; j < W; j++) rows[threadIdx.x * W + j] = v[j];
-            __syncthreads();
-            for (int e = threadIdx.x; e < kLlrThreads * W / 4; e += kLlrThreads)
-                reinterpret_cast<uint4*>(out + base * W)[e] = reinterpret_cast<const uint4*>(rows)[e];
-            __syncthreads();
+    if constexpr ((W & (W - 1)) == 0) {
+        if (wide) {
+            if (idx < count) store_words<W>(out + idx * W, v);
             return;
         }
-    } else if (wide) {
-        if (idx < count) store_words<W>(out + idx * W, v);
+    }
+    if constexpr (CROSS && W >= 6) {
+        static_assert(NARROW == 2 && W % 2 == 0, "FP32 rows");
+        __shared__ __align__(16) uint32_t rows[kLlrThreads * W];
+#pragma unroll
+        for (int j = 0; j < W; j += 2)
+            *reinterpret_cast<uint2*>(rows + threadIdx.x * W + j) = make_uint2(v[j], v[j + 1]);
+        __syncthreads();
+        uint32_t* dst = out + base * W;
+        if (wide && base + kLlrThreads <= count) {
+            for (int e = threadIdx.x; e < kLlrThreads * W / 4; e += kLlrThreads)
+                reinterpret_cast<uint4*>(dst)[e] = reinterpret_cast<const uint4*>(rows)[e];
+        } else {
+            const int words = (int)min((long)kLlrThreads, count - base) * W;
+            for (int e = 2 * threadIdx.x; e < words; e += 2 * kLlrThreads)
+                *reinterpret_cast<uint2*>(dst + e) = *reinterpret_cast<const uint2*>(rows + e);
+        }
+        __syncthreads();
         return;
     }
     if (idx >= count) return;
@@ -628,21 +647,22 @@ __device__ __forceinline__ void write_rows(uint32_t* out, long base, int count, 
     }
 }
 
-template <int N>
+// U: symbols of a thread, 256 apart.
+template <int N, int U>
 __global__ void __launch_bounds__(kLlrThreads) llr_f16_kernel(const __half2* in, const float* ni, __half* out, int count,
                                                                bool wide, PamLut lut) {
     wait_previous();
-    __half2 v[kLlrPerThread];
-    float nv[kLlrPerThread];
-    const long base = (long)blockIdx.x * kLlrThreads * kLlrPerThread;
+    __half2 v[U];
+    float nv[U];
+    const long base = (long)blockIdx.x * kLlrThreads * U;
 #pragma unroll
-    for (int u = 0; u < kLlrPerThread; u++) {
+    for (int u = 0; u < U; u++) {
         const long at = min(base + u * kLlrThreads + (long)threadIdx.x, (long)count - 1);
         v[u] = in[at];
         nv[u] = ni[at];
     }
 #pragma unroll
-    for (int u = 0; u < kLlrPerThread; u++) {
+    for (int u = 0; u < U; u++) {
         float o[2 * N];
         pam_llr<N>(__low2float(v[u]), __high2float(v[u]), nv[u], lut, o);
         uint32_t w[N];
@@ -651,23 +671,23 @@ __global__ void __launch_bounds__(kLlrThreads) llr_f16_kernel(const __half2* in,
             const __half2 h = __floats2half2_rn(o[2 * j], o[2 * j + 1]);
             w[j] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        write_rows<N, 1>(reinterpret_cast<uint32_t*>(out), base + u * kLlrThreads, count, w, wide);
+        write_rows<N, 1, (U > 1)>(reinterpret_cast<uint32_t*>(out), base + u * kLlrThreads, count, w, wide);
     }
 }
 
 // noiseInv index = symbol / symsPerNoise: the block's first quotient by one
 // division, the rest from it (rcp = floor(2^32 / symsPerNoise) + 1, exact
 // while symsPerNoise <= 1024; a larger count changes at most once in a block).
-template <int N>
+template <int N, int U>
 __global__ void __launch_bounds__(kLlrThreads) llr_f32_kernel(const cf* in, const float* ni, float* out, int count,
                                                                int symsPerNoise, unsigned rcp, bool wide, PamLut lut) {
     wait_previous();
-    cf v[kLlrPerThread];
-    float nv[kLlrPerThread];
-    const long base = (long)blockIdx.x * kLlrThreads * kLlrPerThread;
+    cf v[U];
+    float nv[U];
+    const long base = (long)blockIdx.x * kLlrThreads * U;
     const int q0 = (int)(base / symsPerNoise);
 #pragma unroll
-    for (int u = 0; u < kLlrPerThread; u++) {
+    for (int u = 0; u < U; u++) {
         const long at = min(base + u * kLlrThreads + (long)threadIdx.x, (long)count - 1);
         const unsigned r = (unsigned)(at - (long)q0 * symsPerNoise);
         const int q = q0 + (symsPerNoise == 1 ? (int)r
@@ -677,13 +697,13 @@ __global__ void __launch_bounds__(kLlrThreads) llr_f32_kernel(const cf* in, cons
         nv[u] = ni[q];
     }
 #pragma unroll
-    for (int u = 0; u < kLlrPerThread; u++) {
+    for (int u = 0; u < U; u++) {
         float o[2 * N];
         pam_llr<N>(v[u].x, v[u].y, nv[u], lut, o);
         uint32_t w[2 * N];
 #pragma unroll
         for (int j = 0; j < 2 * N; j++) w[j] = __float_as_uint(o[j]);
-        write_rows<2 * N, 2>(reinterpret_cast<uint32_t*>(out), base + u * kLlrThreads, count, w, wide);
+        write_rows<2 * N, 2, (U > 1)>(reinterpret_cast<uint32_t*>(out), base + u * kLlrThreads, count, w, wide);
     }
 }
 
@@ -802,20 +822,42 @@ static int launch_coef_apply(const cf* C, const cf* Y, cf* O, int nSC, int nSym,
 
 // Whether rows of `words` 4-byte LLR words may be stored whole (write_rows).
 static bool llr_wide(const void* out, int words) {
-    const uintptr_t need = words == 6 || words == 3 ? 16 : 4 * (uintptr_t)words;
-    return ((uintptr_t)out & (need - 1)) == 0;
+    const uintptr_t need = words == 6 ? 16 : 4 * (uintptr_t)words;
+    return (uintptr_t)out % need == 0;
 }
 
+// Blocks of a demapper launch with U symbols a thread.
+static unsigned llr_blocks(int N, int U) { return ((unsigned)N + kLlrThreads * U - 1) / (kLlrThreads * U); }
+static bool llr_large(int N) { return llr_blocks(N, kLlrSymbols) >= (unsigned)sm_count(); }
+
+template <int U>
 static int launch_llr_f32(const cf* in, const float* ni, float* out, int N, int n, int spn, cudaStream_t st) {
     const PamLut lut = pam_lut(n);
-    const unsigned g = ((unsigned)N + kLlrThreads * kLlrPerThread - 1) / (kLlrThreads * kLlrPerThread);
+    const unsigned g = llr_blocks(N, U);
     const unsigned rcp = spn > 1 ? (unsigned)(0x100000000ull / (unsigned)spn) + 1u : 0u;
     const bool w = llr_wide(out, 2 * n);
     switch (n) {
-        case 1: return launch_after(llr_f32_kernel<1>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
-        case 2: return launch_after(llr_f32_kernel<2>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
-        case 3: return launch_after(llr_f32_kernel<3>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
-        default: return launch_after(llr_f32_kernel<4>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
+        case 1: return launch_after(llr_f32_kernel<1, U>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
+        case 2: return launch_after(llr_f32_kernel<2, U>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
+        case 3: return launch_after(llr_f32_kernel<3, U>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
+        default: return launch_after(llr_f32_kernel<4, U>, g, kLlrThreads, 0, st, in, ni, out, N, spn, rcp, w, lut);
+    }
+}
+static int launch_llr_f32(const cf* in, const float* ni, float* out, int N, int n, int spn, cudaStream_t st) {
+    return llr_large(N) ? launch_llr_f32<kLlrSymbols>(in, ni, out, N, n, spn, st)
+                        : launch_llr_f32<1>(in, ni, out, N, n, spn, st);
+}
+
+template <int U>
+static int launch_llr_f16(const __half2* in, const float* ni, __half* out, int N, int n, cudaStream_t st) {
+    const PamLut lut = pam_lut(n);
+    const unsigned g = llr_blocks(N, U);
+    const bool w = llr_wide(out, n);
+    switch (n) {
+        case 1: return launch_after(llr_f16_kernel<1, U>, g, kLlrThreads, 0, st, in, ni, out, N, w, lut);
+        case 2: return launch_after(llr_f16_kernel<2, U>, g, kLlrThreads, 0, st, in, ni, out, N, w, lut);
+        case 3: return launch_after(llr_f16_kernel<3, U>, g, kLlrThreads, 0, st, in, ni, out, N, w, lut);
+        default: return launch_after(llr_f16_kernel<4, U>, g, kLlrThreads, 0, st, in, ni, out, N, w, lut);
     }
 }
 
@@ -852,6 +894,13 @@ static int prepare_gram() {
     if (!s) s = prepare_one(gram_kernel<LT, false>);
     return s ? s : allow_max_smem<gram_kernel<LT, false>>();
 }
+template <int N>
+static int prepare_llr() {
+    int s = prepare_one(llr_f16_kernel<N, 1>);
+    if (!s) s = prepare_one(llr_f16_kernel<N, kLlrSymbols>);
+    if (!s) s = prepare_one(llr_f32_kernel<N, 1>);
+    return s ? s : prepare_one(llr_f32_kernel<N, kLlrSymbols>);
+}
 int prepare_plain_kernels() {
     int s = prepare_gram<2>();
     if (!s) s = prepare_gram<4>();
@@ -860,14 +909,10 @@ int prepare_plain_kernels() {
     if (!s) s = prepare_plain_mode<kCoef>();
     if (!s) s = prepare_plain_mode<kApply>();
     if (!s) s = prepare_plain_mode<kChain>();
-    if (!s) s = prepare_one(llr_f16_kernel<1>);
-    if (!s) s = prepare_one(llr_f16_kernel<2>);
-    if (!s) s = prepare_one(llr_f16_kernel<3>);
-    if (!s) s = prepare_one(llr_f16_kernel<4>);
-    if (!s) s = prepare_one(llr_f32_kernel<1>);
-    if (!s) s = prepare_one(llr_f32_kernel<2>);
-    if (!s) s = prepare_one(llr_f32_kernel<3>);
-    if (!s) s = prepare_one(llr_f32_kernel<4>);
+    if (!s) s = prepare_llr<1>();
+    if (!s) s = prepare_llr<2>();
+    if (!s) s = prepare_llr<3>();
+    if (!s) s = prepare_llr<4>();
     return s;
 }
 
@@ -896,18 +941,8 @@ extern "C" int aerial_coef_apply(const aerial_cf32* C, const aerial_cf32* Y_rx, 
 extern "C" int aerial_llr(const aerial_ch2* softEst, const float* noiseInv, uint16_t* llrOut, int N, int nPamBits,
                           void* stream) {
     if (!softEst || !noiseInv || !llrOut || N < 1 || nPamBits < 1 || nPamBits > 4) return AERIAL_ERR_INVALID_ARG;
-    const PamLut lut = pam_lut(nPamBits);
-    const unsigned g = ((unsigned)N + kLlrThreads * kLlrPerThread - 1) / (kLlrThreads * kLlrPerThread);
-    cudaStream_t st = to_stream(stream);
-    const __half2* in = (const __half2*)softEst;
-    __half* out = (__half*)llrOut;
-    const bool w = llr_wide(out, nPamBits);
-    switch (nPamBits) {
-        case 1: return launch_after(llr_f16_kernel<1>, g, kLlrThreads, 0, st, in, noiseInv, out, N, w, lut);
-        case 2: return launch_after(llr_f16_kernel<2>, g, kLlrThreads, 0, st, in, noiseInv, out, N, w, lut);
-        case 3: return launch_after(llr_f16_kernel<3>, g, kLlrThreads, 0, st, in, noiseInv, out, N, w, lut);
-        default: return launch_after(llr_f16_kernel<4>, g, kLlrThreads, 0, st, in, noiseInv, out, N, w, lut);
-    }
+    const auto run = llr_large(N) ? launch_llr_f16<kLlrSymbols> : launch_llr_f16<1>;
+    return run((const __half2*)softEst, noiseInv, (__half*)llrOut, N, nPamBits, to_stream(stream));
 }
 
 extern "C" int aerial_llr_f32(const aerial_cf32* softEst, const float* noiseInv, float* llrOut, int N, int nPamBits,

@@ -1,5 +1,6 @@
 """Stage kernels around the sizes where their dispatch changes, bit-identical to
-the oracle: the Gram's copies go subcarrier by subcarrier above 64 pieces."""
+the oracle: the demapper's four symbols a thread begin at a block per SM, the
+Gram's copies go subcarrier by subcarrier above 64 pieces."""
 from __future__ import annotations
 
 import numpy as np
@@ -7,6 +8,27 @@ import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4])
+@pytest.mark.parametrize("extra,spn,shift", [(-1, 14, 0), (0, 1, 0), (1, 11, 2), (255, 14, 4), (1030, 2000, 6)])
+def test_demapper_around_a_block_per_sm(aeq, orc, cuda, n, extra, spn, shift):
+    N = 1024 * (torch.cuda.get_device_properties(0).multi_processor_count - 1) + 1 + extra
+    rng = np.random.default_rng(N + n)
+    soft = (rng.standard_normal(2 * N) * 0.7).astype(np.float32)
+    ni = (10 ** rng.uniform(0, 3, N // spn + 1)).astype(np.float32)
+    size = N * 2 * n
+    buf = torch.full((size + 16,), float("nan"), device=cuda)
+    s16, ni1 = orc.ref_llr_inputs(N, N)
+    buf16 = torch.full((size + 16,), -1, dtype=torch.int16, device=cuda)
+    aeq.llr_f32(torch.from_numpy(soft).to(cuda), torch.from_numpy(ni).to(cuda), buf[shift:shift + size], N, n, spn)
+    aeq.llr(torch.from_numpy(s16.view(np.int16)).to(cuda), torch.from_numpy(ni1).to(cuda), buf16[shift:shift + size],
+            N, n)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(buf[shift:shift + size].cpu().numpy(), orc.llr_f32(soft.view(np.complex64), ni, n, spn))
+    np.testing.assert_array_equal(buf16[shift:shift + size].cpu().numpy().view(np.uint16), orc.llr_f16io(s16, ni1, n))
+    for b, empty in ((buf, torch.isnan), (buf16, lambda t: t == -1)):              # nothing else written
+        assert empty(b[:shift]).all() and empty(b[shift + size:]).all()
 
 
 @pytest.mark.parametrize("shift", [0, 1])
