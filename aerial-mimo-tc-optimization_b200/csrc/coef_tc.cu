@@ -46,10 +46,13 @@ __device__ __forceinline__ float4 ld_pair(const float2* p, int a0, int A, bool i
 // it has in flight: one k-step's three 16-byte loads a lane before their MMAs
 // left HBM at 4.2 TB/s.  8 slots of 1,584 subcarriers, 64 antennas, 8 layers,
 // 14 symbols (154 MB): 37 us, 30 us with four k-steps at a time, 27 us with eight.
+// Up to 8 antennas there is one k-step, and the registers of eight only take
+// room from other warps (3,276 subcarriers x 8 antennas x 4 layers x 14 symbols
+// 2.9 us with eight, 1.9 us with one).
 constexpr int kTcSteps = 8;
 
-// NMT, NNT: 8-layer and 8-symbol tiles.
-template <int NMT, int NNT, bool VEC>
+// NMT, NNT: 8-layer and 8-symbol tiles; STEPS: k-steps loaded together.
+template <int NMT, int NNT, bool VEC, int STEPS>
 __global__ void __launch_bounds__(256) coef_apply_tc_kernel(const float2* C, const float2* Y, float2* O, int nSC, int nSym, int L, int A) {
     wait_previous();
     const int lane = threadIdx.x & 31;
@@ -61,10 +64,10 @@ __global__ void __launch_bounds__(256) coef_apply_tc_kernel(const float2* C, con
         float acc[NMT][NNT][4] = {};
         const float2* Cs = C + sc * (long)L * A;
         const float2* Ys = Y + sc * (long)nSym * A;
-        for (int j0 = 0; j0 < nK; j0 += kTcSteps) {
-            float4 cv[kTcSteps][NMT], yv[kTcSteps][NNT];
+        for (int j0 = 0; j0 < nK; j0 += STEPS) {
+            float4 cv[STEPS][NMT], yv[STEPS][NNT];
 #pragma unroll
-            for (int j = 0; j < kTcSteps; j++) {
+            for (int j = 0; j < STEPS; j++) {
                 const int a0 = 8 * (j0 + j) + 2 * c;       // past A for steps past nK: zeros
 #pragma unroll
                 for (int mt = 0; mt < NMT; mt++)
@@ -74,7 +77,7 @@ __global__ void __launch_bounds__(256) coef_apply_tc_kernel(const float2* C, con
                     yv[j][nt] = ld_pair<VEC>(Ys + (long)(8 * nt + g) * A, a0, A, 8 * nt + g < nSym);
             }
 #pragma unroll
-            for (int j = 0; j < kTcSteps; j++) {
+            for (int j = 0; j < STEPS; j++) {
                 if (j0 + j >= nK) break;
                 uint32_t b[NNT][2];
 #pragma unroll
@@ -110,10 +113,13 @@ __global__ void __launch_bounds__(256) coef_apply_tc_kernel(const float2* C, con
 template <int NMT, int NNT>
 static int launch_tc(const float2* C, const float2* Y, float2* O, int nSC, int nSym, int L, int A, bool vec,
                       cudaStream_t st) {
-    // a warp per subcarrier, at most the two 256-thread blocks an SM holds at a time, twice over
+    // a warp per subcarrier, at most eight blocks an SM: an SM holds one or two at a
+    // time, and later ones start as others finish
     const unsigned blocks = (unsigned)std::min(((long)nSC + 7) / 8, (long)sm_count() * 8);
-    return launch_after(vec ? coef_apply_tc_kernel<NMT, NNT, true> : coef_apply_tc_kernel<NMT, NNT, false>, blocks, 256, 0,
-                        st, C, Y, O, nSC, nSym, L, A);
+    auto kernel = A <= 8 ? (vec ? coef_apply_tc_kernel<NMT, NNT, true, 1> : coef_apply_tc_kernel<NMT, NNT, false, 1>)
+                         : (vec ? coef_apply_tc_kernel<NMT, NNT, true, kTcSteps>
+                                : coef_apply_tc_kernel<NMT, NNT, false, kTcSteps>);
+    return launch_after(kernel, blocks, 256, 0, st, C, Y, O, nSC, nSym, L, A);
 }
 
 }  // namespace aeq

@@ -1,6 +1,8 @@
 """Stage kernels around the sizes where their dispatch changes, bit-identical to
 the oracle: the demapper's four symbols a thread begin at a block per SM, the
-Gram's copies go subcarrier by subcarrier above 64 pieces."""
+Gram's copies go subcarrier by subcarrier above 64 pieces.  The tensor-core
+coef_apply, within its rounding of the oracle, loads one k-step (8 antennas) or
+eight at a time."""
 from __future__ import annotations
 
 import numpy as np
@@ -50,3 +52,22 @@ def test_gram_around_the_flat_copies(aeq, wl, orc, cuda, ant, lay, shift):
         torch.cuda.synchronize()
         np.testing.assert_array_equal(G.cpu().numpy(), orc.gram(vals.numpy(), 0.25, n, ant, lay))
         assert torch.isnan(buf[:2 * shift]).all() and torch.isnan(buf[2 * (shift + n * lay * lay):]).all()
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("ant", [2, 7, 8, 9, 16, 63, 64, 65, 72, 128, 130])
+def test_coef_apply_tc_around_its_k_steps(aeq, orc, cuda, ant, shift):
+    n, L, S = 13, 9, 9
+    v = orc.ref_uniform(7, n * ant * 2 * (L + S), 1.0)
+    C, Y = v[: n * L * ant * 2].view(np.complex64), v[n * L * ant * 2:].view(np.complex64)
+    dev = []
+    for x in (C, Y):
+        t = torch.empty(x.size + 2, dtype=torch.complex64, device=cuda)[shift:shift + x.size]
+        t.copy_(torch.from_numpy(x.copy()))
+        dev.append(t)
+    O = torch.full((n * L * S,), float("nan"), dtype=torch.complex64, device=cuda)
+    aeq.coef_apply_tc(dev[0], dev[1], O, n, S, L, ant)
+    torch.cuda.synchronize()
+    # both sum the same exact FP16 products in FP32, in another order: ant complex products of size <= 1/2 each
+    np.testing.assert_allclose(O.cpu().numpy(), orc.coef_apply_v2_model(C, Y, n, S, L, ant), rtol=0,
+                               atol=2 * ant * 2.0 ** -23 * max(1.0, ant / 8))
