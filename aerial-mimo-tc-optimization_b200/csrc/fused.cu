@@ -1922,10 +1922,13 @@ namespace aeq {
 // one length, and what they cost is known better than by an item count: the
 // rounds, half of whose last one is free because fewer warps share the memory,
 // times a group's items, two more for each subcarrier's results and six for
-// the solve.  The size of least cost is 1 % off the best of 1, 2, 3, 4, 6 and 8
-// over 442 such launches, 12 items a group 3.5 % and up to 28 % (32 slots of
-// 132 PRB x 160 antennas x 16 layers 510 us at 1, 420 us at 2; 4 of 132 x 160 x 8
-// with BF16X3 operands 49 and 39 us at 1 and 4), 4 everywhere 13 %.
+// the solve; of complex half, whose items are half the bytes, ten for the solve
+// and its results together (4 cells of 132 PRB x 256 antennas x 16 layers 58 us
+// with the others' numbers, which choose 1, and 52 us).  The size of least cost
+// is 1 % off the best of 1, 2, 3, 4, 6 and 8 over 442 such launches, 12 items a
+// group 3.5 % and up to 28 % (32 slots of 132 PRB x 160 antennas x 16 layers 510 us
+// at 1, 420 us at 2; 4 of 132 x 160 x 8 with BF16X3 operands 49 and 39 us at 1 and
+// 4), 4 everywhere 13 %.
 constexpr int kMaxItems = 16, kRoundItems = 12;
 
 // Groups of `fixed` subcarriers, or of about `items` items (fill: see above).
@@ -1971,7 +1974,8 @@ void set_groups(FusedParams& p, int cap, long warps, int prec) {
         for (int gs : {1, 2, 3, 4, 6}) {
             if (gs > cap || gs > 32 / LT) break;
             const long groups = assign_groups(p, 0, gs, cap);
-            const double cost = ((groups + warps - 1) / warps + (double)groups / warps) * (gs * (nChunk + 2) + 6);
+            const int length = p.fmt == AERIAL_FMT_CF16 ? gs * nChunk + 10 : gs * (nChunk + 2) + 6;
+            const double cost = ((groups + warps - 1) / warps + (double)groups / warps) * length;
             if (gs == 1 || cost < least) {
                 best = gs;
                 least = cost;
