@@ -16,15 +16,9 @@ namespace aeq {
 
 using cf = float2;  // {re, im}: the reference's struct cf32 (src/aerial_coef_wmma.cu:60)
 
-// Status helper: map the last launch error to an ABI status.
-inline int launch_status() {
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? AERIAL_OK : (int)e;
-}
-
 // Status of a runtime call.  A failed call also leaves its error in the
-// calling thread's last-error state, where the next launch check
-// (launch_status) would read it as that launch's own; once returned here it
+// calling thread's last-error state, where a caller that asks for it (torch
+// does after its own launches) would take it for its own; once returned here it
 // is cleared.  Sticky errors (a faulted context) stay, as the runtime keeps
 // them.
 inline int rt_status(cudaError_t e) {
