@@ -1900,23 +1900,23 @@ namespace aeq {
 // different cells groups are made equal in items, not in subcarriers (with
 // four subcarriers a group, one of a 64-antenna cell is four times as long as
 // one of a 16-antenna cell in the same round).  Where even groups of
-// kMaxItems items do not fit the resident warps at once, kRoundItems a group
-// balances the rounds against the solves, whose cost is per group.
+// kMaxItems items do not fit the resident warps at once, the launch takes several
+// rounds, and what they cost depends on how full the last one is and on which
+// cells' groups meet in one warp: of some sizes, that whose longest warp has the
+// least to do is taken, in items with kSolveItems for each solve.
 //
 // Measured back to back, subcarriers per group 4 everywhere -> this rule:
 // one slot of 24 PRB x 32 antennas x 4 layers 8.3 -> 6.3 us, two of
 // 132 x 64 x 8 16.5 -> 14.5, one of 100 PRB x 48 x 3 16.5 -> 10.4; mixed
-// batches of 8 / 16 / 48 cells 32.9 -> 27 / 34 -> 33 / 112 -> 103 us, of 24
-// and 48 cells with ragged shapes 72 -> 53 and 114 -> 106 us.  8 or 16 items in
-// the rounds' place are 1 % slower over mixed batches.  One subcarrier a group
-// in a uniform batch keeps most lanes of the solve idle and pays only while half
-// the warps are free (one slot of 132 x 64 x 8: 10.9 us at 1, 10.3 us at 2).
+// batches of 8 cells 32.9 -> 27 us.  In rounds, over 154 mixed batches of 8 to 64
+// cells: 2.5 % off the best of ten sizes (geometric mean), 12 items everywhere
+// 4.6 %, 16 items 4.9 %, four subcarriers 9.4 %.  The 16 uneven cells of the
+// benchmark, L2 flushed: 53.4 us with four subcarriers, 56.1 us with 12 items,
+// 52.4 us; in complex half 45.5, 47.6 and 43.4 us.  Choosing takes the host 1.2 us
+// for 16 cells, 6 us for 64.  One subcarrier a group in a uniform batch keeps most
+// lanes of the solve idle and pays only while half the warps are free (one slot of
+// 132 x 64 x 8: 10.9 us at 1, 10.3 us at 2).
 // A subcarrier's results do not depend on its group.
-//
-// In rounds, a group of full layers that leaves a quarter of its solve's lanes
-// idle or less is made a full one (three subcarriers of 8 layers become four):
-// 12 / 24 / 48 uneven cells 40 -> 37, 51 -> 49 and 113 -> 107 us; not with split
-// operands, whose items cost more (24 uneven cells, BF16X3: 57 and 58 us).
 //
 // Cells of one tile and chunk count (outside the uniform kernels) have groups of
 // one length, and what they cost is known better than by an item count: the
@@ -1929,17 +1929,15 @@ namespace aeq {
 // group 3.5 % and up to 28 % (32 slots of 132 PRB x 160 antennas x 16 layers 510 us
 // at 1, 420 us at 2; 4 of 132 x 160 x 8 with BF16X3 operands 49 and 39 us at 1 and
 // 4), 4 everywhere 13 %.
-constexpr int kMaxItems = 16, kRoundItems = 12;
+constexpr int kMaxItems = 16, kSolveItems = 8;
 
-// Groups of `fixed` subcarriers, or of about `items` items (fill: see above).
-static long assign_groups(FusedParams& p, int items, int fixed, int cap, bool fill = false) {
+// Groups of `fixed` subcarriers, or of about `items` items.
+static long assign_groups(FusedParams& p, int items, int fixed, int cap) {
     long g0 = 0;
     for (int i = 0; i < p.nCells; i++) {
         FusedCell& f = p.cell[i];
-        const int lanes = 32 / f.LT;
-        const int most = lanes < cap ? lanes : cap;
-        int gs = fixed ? fixed : (items + f.nChunk / 2) / f.nChunk;
-        if (fill && f.exact && 4 * gs >= 3 * lanes) gs = lanes;
+        const int most = 32 / f.LT < cap ? 32 / f.LT : cap;
+        const int gs = fixed ? fixed : (items + f.nChunk / 2) / f.nChunk;
         f.GS = gs < 1 ? 1 : gs > most ? most : gs;
         f.group0 = g0;
         g0 += (f.nSC + f.GS - 1) / f.GS;
@@ -1948,7 +1946,33 @@ static long assign_groups(FusedParams& p, int items, int fixed, int cap, bool fi
     return g0;
 }
 
-void set_groups(FusedParams& p, int cap, long warps, int prec) {
+// The load of the warp that has most, warp w holding groups w, w + warps, ...:
+// warp 0's, and from there the steps where, in some round, one cell's groups end
+// and the next one's begin.
+static int longest_warp(const FusedParams& p, unsigned warps) {
+    uint64_t step[kMaxCells];                         // warp << 32 | step + 2^31: in order of the warps
+    int n = 0, cost = p.cell[0].GS * p.cell[0].nChunk + kSolveItems, load = 0;
+    unsigned rounds = 0;                              // rounds begun by the cells so far
+    for (int i = 0; i < p.nCells; i++) {
+        const bool last = i + 1 == p.nCells;
+        const unsigned end = (unsigned)(last ? p.totalGroups : p.cell[i + 1].group0), q = end / warps, at = end - q * warps;
+        const unsigned begun = q + (at != 0);
+        load += cost * (int)(begun - rounds);
+        rounds = begun;
+        const int next = last ? 0 : p.cell[i + 1].GS * p.cell[i + 1].nChunk + kSolveItems;
+        if (at) step[n++] = (uint64_t)at << 32 | (uint32_t)(next - cost + INT32_MIN);
+        cost = next;
+    }
+    std::sort(step, step + n);
+    int longest = load;
+    for (int k = 0; k < n; k++) {
+        load += (int)((uint32_t)step[k] - (uint32_t)INT32_MIN);
+        if (k + 1 == n || step[k + 1] >> 32 != step[k] >> 32) longest = std::max(longest, load);
+    }
+    return longest;
+}
+
+void set_groups(FusedParams& p, int cap, long warps) {
     if (cap >= kFullGroups) {
         assign_groups(p, 0, kFullGroups, kFullGroups);
         return;
@@ -1987,7 +2011,17 @@ void set_groups(FusedParams& p, int cap, long warps, int prec) {
     if (subcarriers <= warps * cap)                   // else no grouping fits one round
         for (int items : {1, 2, 3, 4, 5, 6, 8, 10, 12, kMaxItems})
             if (assign_groups(p, items, 0, cap) <= warps) return;
-    assign_groups(p, kRoundItems, 0, cap, prec == AERIAL_PREC_FP16 || prec == AERIAL_PREC_BF16);
+    int best = kMaxItems, least = INT32_MAX;
+    for (int items : {10, 12, 14, 16, 20, 24}) {
+        if (warps < 1) break;                         // no launch will come of it
+        assign_groups(p, items, 0, cap);
+        const int load = longest_warp(p, (unsigned)warps);
+        if (load < least) {
+            best = items;
+            least = load;
+        }
+    }
+    assign_groups(p, best, 0, cap);
 }
 
 // warpBytes: the per-warp shared memory of the launch (epilogue region of the
@@ -2439,7 +2473,7 @@ extern "C" int aerial_pusch_eq_fused(const aerial_cell_desc* cells, int nCells, 
     LaunchShape sh;
     int prec, gsCap;
     resolve_tuning(tuning, warpBytes, prec, sh, gsCap);
-    set_groups(p, gsCap, resident_warps(sh), prec);
+    set_groups(p, gsCap, resident_warps(sh));
     set_operand_scale(p, prec);
     return launch_fused(p, warpBytes, prec, sh, to_stream(stream));
 }
@@ -2479,7 +2513,7 @@ extern "C" int aerial_autotune(const aerial_cell_desc* cells, int nCells, aerial
         int gs[3][kMaxCells];
         for (int ic = 0; ic < nCaps; ic++) {
             p = base;
-            set_groups(p, caps[ic], resident_warps(sh), prec);
+            set_groups(p, caps[ic], resident_warps(sh));
             bool seen = false;
             for (int i = 0; i < p.nCells; i++) gs[ic][i] = p.cell[i].GS;
             for (int k = 0; k < ic && !seen; k++) seen = std::equal(gs[k], gs[k] + p.nCells, gs[ic]);
@@ -2508,7 +2542,7 @@ extern "C" int aerial_autotune(const aerial_cell_desc* cells, int nCells, aerial
         for (int ic = 0; ic < nc && !s; ic++) {
             const LaunchShape& sh = cand[ic].sh;
             p = base;                                // unscaled sigma2
-            set_groups(p, cand[ic].cap, resident_warps(sh), prec);
+            set_groups(p, cand[ic].cap, resident_warps(sh));
             set_operand_scale(p, prec);
             if ((s = launch_fused(p, warpBytes, prec, sh, st))) break;
             cudaEventRecord(e0, st);
@@ -2600,7 +2634,7 @@ extern "C" int aerial_eq_graph_create(const aerial_cell_desc* cells, int nCells,
     int s = build_fused_params(cells, nCells, g->params, warpBytes);
     if (!s) {
         resolve_tuning(tuning, warpBytes, g->prec, g->shape, g->gsCap);
-        set_groups(g->params, g->gsCap, resident_warps(g->shape), g->prec);
+        set_groups(g->params, g->gsCap, resident_warps(g->shape));
         set_operand_scale(g->params, g->prec);
         s = plan_fused(g->params, warpBytes, g->prec, g->shape, g->plan);
     }
@@ -2653,7 +2687,7 @@ extern "C" int aerial_eq_graph_update(aerial_eq_graph* g, const aerial_cell_desc
     // The new noise levels may move a cell in or out of FP16 operand scaling,
     // which selects another kernel instantiation: re-plan the node (an
     // executable graph's kernel node may change its function).
-    set_groups(np, g->gsCap, resident_warps(g->shape), g->prec);
+    set_groups(np, g->gsCap, resident_warps(g->shape));
     set_operand_scale(np, g->prec);
     np.walkSlot = g->params.walkSlot;
     LaunchPlan pl;
