@@ -187,7 +187,8 @@ __device__ __forceinline__ float2 sub_bf16(uint32_t h, float re, float im) {
     return d;
 }
 // bf16 hi/lo split of a complex pair: x = hi + lo to ~16 mantissa bits.  The
-// same bits either way.
+// same values either way (from the halves, a remainder of zero is -0, which no
+// sum of products shows).
 template <bool HALVES>
 __device__ __forceinline__ void split_bf16(float re, float im, uint32_t& hi, uint32_t& lo) {
     __nv_bfloat162 h = __floats2bfloat162_rn(re, im), l;
@@ -2373,11 +2374,8 @@ static WalkTable* walk_table_locked(std::unique_lock<std::mutex>& lk, int* devOu
 }
 
 // The unrolled kernels (uniform batches) take the dynamic walk: they ask for
-// their next group a subcarrier ahead of needing it.  The mixed-tile kernels'
-// producer cursor would ask at the moment it stages the group, and on the
-// uneven 16-cell batch that measured slower (57.4-58.2 against 54.3 us; with
-// the ticket taken a whole group ahead still 58.4 against 54.2 us), so they
-// keep the static walk.
+// their next group a subcarrier ahead of needing it.  The others keep a fixed
+// assignment, by which set_groups chooses their groups' sizes.
 // A launch whose warps hold one group each at most never asks for a ticket.
 static bool walk_applies(const FusedParams& p, const LaunchPlan& pl) {
     return p.exactChunks != 0 && !p.halfMixed && p.totalGroups > (long)pl.grid.x * (pl.block.x / 32);

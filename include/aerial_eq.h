@@ -15,7 +15,8 @@
  *   - `stream` is a cudaStream_t passed as void* (NULL = legacy default
  *     stream).  Work is enqueued asynchronously on it, behind everything
  *     enqueued before (kernels are launched with programmatic stream
- *     serialization and wait for the stream on the device).
+ *     serialization and wait for the stream on the device; captured into a
+ *     graph, a kernel behind another one has a programmatic edge).
  *   - Return value: AERIAL_OK (0), an AERIAL_ERR_* code for bad arguments,
  *     or a cudaError_t value (1..999) from the launch.  Nothing calls
  *     exit(); the reference's CUDA_CHECK -> exit(1) becomes a status.

@@ -70,3 +70,26 @@ def test_outputs_over_inputs(aeq, wl, orc, cuda, over, static):
     np.testing.assert_array_equal(llr.cpu().numpy(), l)
     np.testing.assert_array_equal(yeq.cpu().numpy(), y)
     np.testing.assert_array_equal(lo.cpu().numpy(), _oracle(orc, other.H.numpy(), other.Y.numpy(), other)[0])
+
+
+def test_static_calls_overlap(aeq, wl, orc, cuda):
+    """Calls on two streams at a time share nothing; each gives the oracle's results."""
+    cells = [wl.make_cell(132, 64, 8, 11, 256, 25.0, seed=920), wl.make_cell(51, 32, 3, 7, 16, 20.0, seed=921)]
+    ref = [_oracle(orc, c.H.numpy(), c.Y.numpy(), c) for c in cells]
+    streams = [torch.cuda.Stream() for _ in cells]
+    runs = []
+    for c in cells:
+        H, Y = c.H.to(cuda), c.Y.to(cuda)
+        n = c.nSC * c.nLayers * c.nSym
+        outs = [(torch.full((c.llr_numel,), float("nan"), device=cuda),
+                 torch.full((n,), float("nan"), dtype=torch.complex64, device=cuda)) for _ in range(6)]
+        runs.append([(o, _desc(aeq, c, H, Y, *o)) for o in outs])
+    torch.cuda.synchronize()
+    for step in zip(*runs):
+        for (_, d), s in zip(step, streams):
+            aeq.pusch_eq_plain_static([d], s)
+    torch.cuda.synchronize()
+    for (l, y), calls in zip(ref, runs):
+        for (llr, yeq), _ in calls:
+            np.testing.assert_array_equal(llr.cpu().numpy(), l)
+            np.testing.assert_array_equal(yeq.cpu().numpy(), y)
